@@ -72,14 +72,16 @@ extern "C" int ms_gpu_arena_create(uint64_t cap, ms_arena **out) {
     if (!out || cap == 0) return ms_fail(MS_ERR_INVALID, "arena_create: bad argument");
     ms_arena *a = new ms_arena();
     MS_CUDA_TRY(cudaGetDevice(&a->device));
-    cudaError_t e = cudaMalloc(&a->base, cap + 256);
+    // the error word sits behind the bump range, aligned whatever the capacity
+    const uint64_t err_off = ms::align_up(cap, 256);
+    cudaError_t e = cudaMalloc(&a->base, err_off + 256);
     if (e != cudaSuccess) {
         delete a;
         return ms_fail_cuda(e, "arena cudaMalloc");
     }
     a->cap = cap;
     a->used = 0;
-    a->d_err = reinterpret_cast<unsigned *>(a->base + cap);  // tail word, outside the bump range
+    a->d_err = reinterpret_cast<unsigned *>(a->base + err_off);
     MS_CUDA_TRY(cudaMemset(a->d_err, 0, 256));
     *out = a;
     return MS_OK;

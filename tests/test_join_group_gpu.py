@@ -159,3 +159,16 @@ def test_natural_join_hash_path_and_edges(ms, arena, orc):
         ol, orr = ms.natural_join(a, b)
         assert ol.get_count_values() == 0 and orr.get_count_values() == 0
 
+
+
+def test_group_in_an_arena_of_odd_size(ms, orc):
+    """Kernels report through the arena's error word, which has to be aligned
+    whatever the arena's capacity (the group table grows through it)."""
+    v = orc.uniform_bits(3, 16, 60_001)
+    a = ms.Arena((64 << 20) + 1)
+    try:
+        gr, ext = ms.group(ms.Column.from_numpy(v, a))
+        egr, eext = orc.group(v)
+        assert np.array_equal(gr.to_numpy(), egr) and np.array_equal(ext.to_numpy(), eext)
+    finally:
+        a.close()
