@@ -172,3 +172,30 @@ def test_group_in_an_arena_of_odd_size(ms, orc):
         assert np.array_equal(gr.to_numpy(), egr) and np.array_equal(ext.to_numpy(), eext)
     finally:
         a.close()
+
+
+@pytest.mark.parametrize("groups", [1, 31, 2047, 2048, 2049, 4096, 4097, 9001, 24576, 24577, 40_000])
+@pytest.mark.parametrize("fmt", [O.UNCOMPR, O.DYNAMIC_VBP])
+def test_group_counts_around_table_limits(ms, arena, orc, groups, fmt):
+    """Group counts at the edges of the shared-memory tables, of the ranked
+    list and of the first global table; sums of 64-bit values, which carry
+    and wrap.  The rows of one key are spread, and 2^64 - 1 is a key."""
+    n = 2 * groups + 3 * 4096 + 5
+    keys = orc.uniform_bits(groups, 64 if fmt == O.UNCOMPR else 40, groups)
+    keys[-1] = np.uint64((1 << 64) - 1 if fmt == O.UNCOMPR else 7)
+    pick = orc.uniform_bits(groups + 1, 32, n) % np.uint64(groups)
+    pick[orc.uniform_bits(groups + 2, 63, n).argsort(kind="stable")[:groups]] = np.arange(groups, dtype=np.uint64)
+    v = keys[pick.astype(np.int64)]
+    m = orc.uniform_bits(groups + 3, 64, n)
+    egr, eext = orc.group(v)
+    gr, ext = ms.group(_col(ms, arena, orc, v, fmt))
+    assert np.array_equal(ext.to_numpy(), eext)
+    assert np.array_equal(gr.to_numpy(), egr)
+    s = ms.agg_sum_grouped(gr, ms.Column.from_numpy(m, arena), len(eext))
+    assert np.array_equal(s.to_numpy(), orc.agg_sum_grouped(egr, m, len(eext)))
+    # binary group: (first grouping, another key)
+    k2 = orc.uniform_bits(groups + 4, 3, n)
+    gr2, ext2 = ms.group(ms.Column.from_numpy(k2, arena), gr)
+    egr2, eext2 = orc.group(k2, egr)
+    assert np.array_equal(ext2.to_numpy(), eext2)
+    assert np.array_equal(gr2.to_numpy(), egr2)
