@@ -89,25 +89,6 @@ __device__ __forceinline__ bool cmp_bits(uint64_t v, uint64_t c, unsigned cf, bo
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// Threshold form of `base + d  cmp  c` (signed 64-bit, as the compressed
-// part compares) for d in [0, range), range <= 2^32: a Pred on d.  False when
-// base + [0, range) wraps or crosses the signed boundary -- then the order of
-// d is not the order of the values and the caller compares 64-bit values.
-__device__ __forceinline__ bool rel_pred(uint64_t base, uint64_t range, uint64_t c, int cmp, Pred &p) {
-    const uint64_t hi = base + (range - 1);
-    if (hi < base || ((int64_t)base < 0) != ((int64_t)hi < 0)) return false;
-    const int64_t cs = (int64_t)c, bs = (int64_t)base;
-    const uint64_t diff = uint64_t(cs) - uint64_t(bs);  // the true difference when cs >= bs
-    const uint64_t nlt = cs <= bs ? 0 : minu(diff, range);
-    const uint64_t nle = cs < bs ? 0 : (diff >= range ? range : diff + 1);
-    p.cmp = cmp;
-    p.val = c - base;
-    p.is_eq = cmp == MS_CMP_EQ;
-    p.T = (cmp == MS_CMP_LT || cmp == MS_CMP_GE) ? nlt : nle;
-    p.flip = cmp == MS_CMP_GT || cmp == MS_CMP_GE;
-    return true;
-}
-
 // A delta_f block of width BW <= 27 in 32-bit arithmetic: thread (l, q)
 // decodes its 16 deltas, forms their running sums P_k (< 2^31), and the
 // lane's values are base + P_k with base = carry + the sums of the lane's

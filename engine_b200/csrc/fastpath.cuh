@@ -41,6 +41,25 @@ inline Pred make_pred(int cmp, uint64_t c) {
     return p;
 }
 
+// Threshold form of `base + d  cmp  c` (signed 64-bit, as the compressed
+// part compares) for d in [0, range), range <= 2^32: a Pred on d.  False when
+// base + [0, range) wraps or crosses the signed boundary -- then the order of
+// d is not the order of the values and the caller compares 64-bit values.
+__device__ __forceinline__ bool rel_pred(uint64_t base, uint64_t range, uint64_t c, int cmp, Pred &p) {
+    const uint64_t hi = base + (range - 1);
+    if (hi < base || ((int64_t)base < 0) != ((int64_t)hi < 0)) return false;
+    const int64_t cs = (int64_t)c, bs = (int64_t)base;
+    const uint64_t diff = uint64_t(cs) - uint64_t(bs);  // the true difference when cs >= bs
+    const uint64_t nlt = cs <= bs ? 0 : minu(diff, range);
+    const uint64_t nle = cs < bs ? 0 : (diff >= range ? range : diff + 1);
+    p.cmp = cmp;
+    p.val = c - base;
+    p.is_eq = cmp == MS_CMP_EQ;
+    p.T = (cmp == MS_CMP_LT || cmp == MS_CMP_GE) ? nlt : nle;
+    p.flip = cmp == MS_CMP_GT || cmp == MS_CMP_GE;
+    return true;
+}
+
 // 16 values of quarter q of lane l as 32-bit integers (bw <= 32).
 template <unsigned BW>
 __device__ __forceinline__ void vbp_decode16_u32(const uint64_t *__restrict__ blk, unsigned l, unsigned q,
@@ -199,6 +218,21 @@ __device__ __forceinline__ uint64_t sum_block_rt(unsigned bw, const uint64_t *bl
         MS_BW_CASES(MS_X)
 #undef MS_X
     default: bad = true; return 0;
+    }
+}
+
+// 16 values of a block of width 1..32 as 32-bit integers; false for other
+// widths.
+__device__ __forceinline__ bool vbp_decode16_u32_rt(unsigned bw, const uint64_t *blk, unsigned l, unsigned q,
+                                                    uint32_t (&v)[16]) {
+    switch (bw) {
+#define MS_X(B) \
+    case B: vbp_decode16_u32<B>(blk, l, q, v); return true;
+        MS_X(1) MS_X(2) MS_X(3) MS_X(4) MS_X(5) MS_X(6) MS_X(7) MS_X(8) MS_X(9) MS_X(10) MS_X(11) MS_X(12)
+        MS_X(13) MS_X(14) MS_X(15) MS_X(16) MS_X(17) MS_X(18) MS_X(19) MS_X(20) MS_X(21) MS_X(22) MS_X(23)
+        MS_X(24) MS_X(25) MS_X(26) MS_X(27) MS_X(28) MS_X(29) MS_X(30) MS_X(31) MS_X(32)
+#undef MS_X
+    default: return false;
     }
 }
 

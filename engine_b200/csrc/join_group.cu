@@ -3,7 +3,7 @@
 //
 // Membership (semi_join build side): when the build keys span at most 2^27
 // values the set is a dense bitmap (exact, one bit per value; kept in
-// shared memory when it fits 128 KB), otherwise an open-addressing hash set
+// shared memory when it fits 208 KB), otherwise an open-addressing hash set
 // in global memory (linear probing, 64-bit multiplicative hash).  The
 // reference uses a vectorised linear-probing hash set
 // (vector/datastructures/hash_based/hash_set.h:32-149); results do not
@@ -15,6 +15,7 @@
 // (linear_probing.h:437-443, scalar/group_uncompr.h:105-114) -- and the
 // flagged rows in order are the group extents.
 #include "internal.h"
+#include "positions.cuh"
 #include "scan.cuh"
 
 namespace ms {
@@ -64,27 +65,6 @@ __device__ __forceinline__ bool set_contains(const KeySet &s, const uint32_t *sb
     return false;
 }
 
-__global__ void k_minmax(ColView c, unsigned long long *mn, unsigned long long *mx, unsigned *err) {
-    const unsigned lane = threadIdx.x & 31u, l = lane & 7u, q = lane >> 3;
-    uint64_t lo = kEmpty, hi = 0;
-    bool ok = true;
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < c.nblocks_total();
-         b += uint64_t(gridDim.x) * blockDim.x / 32) {
-        uint64_t v[16];
-        unsigned valid;
-        ok &= decode_block(c, b, l, q, v, valid);
-#pragma unroll
-        for (int k = 0; k < 16; k++)
-            if ((valid >> k) & 1u) {
-                lo = minu(lo, v[k]);
-                hi = maxu(hi, v[k]);
-            }
-    }
-    if (!ok) atomicOr(err, kErrCorrupt);
-    atomicMin(mn, (unsigned long long)lo);
-    atomicMax(mx, (unsigned long long)hi);
-}
-
 __global__ void k_build_set(ColView c, uint32_t *bits, uint64_t lo, uint64_t *slots, uint64_t mask,
                             int *has_max, unsigned *err) {
     const unsigned lane = threadIdx.x & 31u, l = lane & 7u, q = lane >> 3;
@@ -124,50 +104,60 @@ __global__ void k_build_set(ColView c, uint32_t *bits, uint64_t lo, uint64_t *sl
     if (!ok) atomicOr(err, kErrCorrupt);
 }
 
-// Probe: per block, hits = rows of r whose value is in the set.  Pass 1
-// (blk_off == nullptr) stores per-block counts, pass 2 writes positions.
-constexpr unsigned kSmemBitmapWords = 32768;  // 128 KB
+// Probe, pass 1: hit bits = rows of r whose value is in the set.  A bitmap of
+// up to kSmemBitmapWords is copied into shared memory by one CTA of 24 warps
+// per SM (random words of global memory cost one L1 line each, 32 per warp
+// load; shared memory serves them at its bank conflicts).  Blocks of width <=
+// 32 are decoded to 32-bit values; a value's place in the bitmap is its
+// distance from the smallest key, which is at or beyond the span for any
+// value below that key.
+constexpr unsigned kSmemBitmapWords = 53248;  // 208 KB
+constexpr unsigned kProbeWarps = 24;
 
 template <bool kSmem>
-__global__ void __launch_bounds__(256) k_probe(ColView r, KeySet s, uint32_t *__restrict__ blk_counts,
-                                              const uint64_t *__restrict__ blk_off, uint64_t *__restrict__ out_pos,
-                                              unsigned long long *__restrict__ d_scalar_hits, unsigned *err) {
+__global__ void __launch_bounds__(kSmem ? 32 * kProbeWarps : 256, kSmem ? 1 : 3)
+    k_probe_bits(ColView r, KeySet s, MaskRun run, unsigned *err) {
     extern __shared__ uint32_t sbits[];
     if (kSmem) {
-        const uint64_t words = (s.span + 31) / 32;
-        for (uint64_t i = threadIdx.x; i < words; i += blockDim.x) sbits[i] = s.bits[i];
+        const uint32_t words = uint32_t((s.span + 31) / 32);
+        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) sbits[i] = __ldg(s.bits + i);
         __syncthreads();
     }
-    const unsigned lane = threadIdx.x & 31u, l = lane & 7u, q = lane >> 3;
     bool ok = true;
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < r.nblocks_total();
-         b += uint64_t(gridDim.x) * blockDim.x / 32) {
+    const bool narrow = s.bits && (r.fmt == MS_FMT_STATIC_VBP || r.fmt == MS_FMT_DYNAMIC_VBP || r.fmt == MS_FMT_FOR_DVBP);
+    mask_pass(run, [&](uint64_t b, unsigned l, unsigned q) -> unsigned {
+        unsigned m = 0;
+        if (narrow && b < r.nb()) {
+            uint64_t off;
+            unsigned bw;
+            if (r.fmt == MS_FMT_STATIC_VBP) {
+                bw = r.bw;
+                off = b * 64ull * bw;
+            } else {
+                const uint64_t e = __ldg(r.index + b);
+                off = idx_off(e);
+                bw = idx_bw(e);
+            }
+            uint32_t v[16];
+            if (vbp_decode16_u32_rt(bw, reinterpret_cast<const uint64_t *>(r.data + off), l, q, v)) {
+                const uint64_t base = (r.fmt == MS_FMT_FOR_DVBP ? __ldg(r.aux + (b >> 1)) : 0) - s.lo;
+#pragma unroll
+                for (int k = 0; k < 16; k++) {
+                    const uint64_t d = base + v[k];
+                    const uint32_t w = d < s.span ? (kSmem ? sbits[uint32_t(d >> 5)] : __ldg(s.bits + (d >> 5))) : 0u;
+                    m |= ((w >> (unsigned(d) & 31u)) & 1u) << k;
+                }
+                return m;
+            }
+        }
         uint64_t v[16];
         unsigned valid;
         ok &= decode_block(r, b, l, q, v, valid);
-        unsigned m = 0;
 #pragma unroll
         for (int k = 0; k < 16; k++)
             if ((valid >> k) & 1u) m |= unsigned(set_contains(s, kSmem ? sbits : nullptr, v[k])) << k;
-        if (!blk_off) {
-            const unsigned tot = __reduce_add_sync(0xFFFFFFFFu, __popc(m));
-            if (lane == 0) blk_counts[b] = tot;
-            continue;
-        }
-        if (!__any_sync(0xFFFFFFFFu, m != 0)) continue;
-        unsigned rank[16];
-        block_ranks(m, l, q, rank);
-        const uint64_t base = blk_off[b], row0 = b * kBlock;
-        unsigned scal = 0;
-#pragma unroll
-        for (int k = 0; k < 16; k++)
-            if ((m >> k) & 1u) {
-                const uint64_t row = row0 + (16u * q + k) * 8u + l;
-                out_pos[base + rank[k]] = row;
-                scal += row >= r.sfrom;
-            }
-        if (scal) atomicAdd(d_scalar_hits, (unsigned long long)scal);
-    }
+        return m;
+    });
     if (!ok) atomicOr(err, kErrCorrupt);
 }
 
@@ -180,7 +170,8 @@ __global__ void __launch_bounds__(256) k_probe(ColView r, KeySet s, uint32_t *__
 // order in which warps insert.
 // ---------------------------------------------------------------------------
 struct KeyMap {
-    unsigned long long *dense;  // dense mode: position per key - lo (~0: absent)
+    uint32_t *dense;      // dense mode: position per key - lo (~0: absent); builds of fewer than 2^32 - 1 rows
+    uint32_t *bits;       // dense mode: keys present
     uint64_t lo, span;
     unsigned long long *keys;   // hash mode
     unsigned long long *vals;
@@ -191,7 +182,9 @@ struct KeyMap {
 __device__ __forceinline__ uint64_t map_lookup(const KeyMap &m, uint64_t k) {
     if (m.dense) {
         const uint64_t d = k - m.lo;
-        return (k < m.lo || d >= m.span) ? kEmpty : m.dense[d];
+        if (d >= m.span) return kEmpty;
+        const uint32_t p = m.dense[d];
+        return p == ~0u ? kEmpty : p;
     }
     if (k == kEmpty) return *m.max_pos;
     uint64_t h = hash64(k) & m.mask;
@@ -218,7 +211,9 @@ __global__ void k_build_map(ColView c, KeyMap m, unsigned *err) {
             const uint64_t key = v[k];
             const unsigned long long row = b * kBlock + (16u * q + k) * 8u + l;
             if (m.dense) {
-                atomicMin(m.dense + (key - m.lo), row);
+                const uint64_t d = key - m.lo;
+                atomicMin(m.dense + d, uint32_t(row));
+                atomicOr(m.bits + (d >> 5), 1u << (d & 31u));
                 continue;
             }
             if (key == kEmpty) {
@@ -242,46 +237,51 @@ __global__ void k_build_map(ColView c, KeyMap m, unsigned *err) {
     if (!ok) atomicOr(err, kErrCorrupt);
 }
 
-// Probe: per block, hits = rows of r whose value is a key.  Pass 1
-// (blk_off == nullptr) stores per-block counts, pass 2 writes the pairs.
-__global__ void __launch_bounds__(256) k_probe_map(ColView r, KeyMap m, uint32_t *__restrict__ blk_counts,
-                                                  const uint64_t *__restrict__ blk_off, uint64_t *__restrict__ out_r,
-                                                  uint64_t *__restrict__ out_l,
-                                                  unsigned long long *__restrict__ d_scalar_hits, unsigned *err) {
-    const unsigned lane = threadIdx.x & 31u, l = lane & 7u, q = lane >> 3;
-    bool ok = true;
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < r.nblocks_total();
-         b += uint64_t(gridDim.x) * blockDim.x / 32) {
-        uint64_t v[16];
-        unsigned valid;
-        ok &= decode_block(r, b, l, q, v, valid);
-        unsigned mk = 0;
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const uint64_t p = ((valid >> k) & 1u) ? map_lookup(m, v[k]) : kEmpty;
-            v[k] = p;  // the build position replaces the value
-            mk |= unsigned(p != kEmpty) << k;
-        }
-        if (!blk_off) {
-            const unsigned tot = __reduce_add_sync(0xFFFFFFFFu, __popc(mk));
-            if (lane == 0) blk_counts[b] = tot;
-            continue;
-        }
-        if (!__any_sync(0xFFFFFFFFu, mk != 0)) continue;
-        unsigned rank[16];
-        block_ranks(mk, l, q, rank);
-        const uint64_t base = blk_off[b], row0 = b * kBlock;
-        unsigned scal = 0;
-#pragma unroll
-        for (int k = 0; k < 16; k++)
-            if ((mk >> k) & 1u) {
-                const uint64_t row = row0 + (16u * q + k) * 8u + l;
-                out_r[base + rank[k]] = row;
-                out_l[base + rank[k]] = v[k];
-                scal += row >= r.sfrom;
-            }
-        if (scal) atomicAdd(d_scalar_hits, (unsigned long long)scal);
+// Probe, pass 1: hit bits = rows of r whose value is a key, and the build
+// positions of a block's hits one after another at side + 512 * block (V:
+// 32 bits while positions fit).  kSmem: the bitmap of present keys in shared
+// memory decides the rows, so that only hits read the position array (one
+// L1 line per row otherwise, which is what bounds a probe of all rows).
+template <bool kSmem, class V>
+__global__ void __launch_bounds__(kSmem ? 32 * kProbeWarps : 256, kSmem ? 1 : 3)
+    k_probe_map_bits(ColView r, KeyMap m, MaskRun run, V *__restrict__ side, unsigned *err) {
+    extern __shared__ uint32_t sbits[];
+    if (kSmem) {
+        const uint32_t words = uint32_t((m.span + 31) / 32);
+        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) sbits[i] = __ldg(m.bits + i);
+        __syncthreads();
     }
+    bool ok = true;
+    mask_pass(run, [&](uint64_t b, unsigned l, unsigned q) -> unsigned {
+        uint64_t v[16];
+        unsigned valid, mk = 0;
+        ok &= decode_block(r, b, l, q, v, valid);
+        V *const o = side + (b - run.b0) * kBlock;
+        if (kSmem) {
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                const uint64_t d = v[k] - m.lo;
+                v[k] = d;
+                if (d < m.span) mk |= ((sbits[uint32_t(d >> 5)] >> (unsigned(d) & 31u)) & 1u) << k;
+            }
+            mk &= valid;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                const uint64_t p = ((valid >> k) & 1u) ? map_lookup(m, v[k]) : kEmpty;
+                v[k] = p;  // the build position replaces the value
+                mk |= unsigned(p != kEmpty) << k;
+            }
+        }
+        if (__any_sync(0xFFFFFFFFu, mk != 0)) {
+            unsigned rank[16];
+            block_ranks(mk, l, q, rank);
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                if ((mk >> k) & 1u) o[rank[k]] = kSmem ? V(__ldg(m.dense + v[k])) : V(v[k]);
+        }
+        return mk;
+    });
     if (!ok) atomicOr(err, kErrCorrupt);
 }
 
@@ -738,6 +738,13 @@ static int positions_two_pass(uint64_t nbt, Launch launch, int out_format, unsig
     return write_values(pos, total - scal, scal, out_format, out_bw, out, a, st);
 }
 
+// The bitmap goes to shared memory when it fits and the probe side is long
+// enough to pay for each SM's copy: an SM copies `words` and then looks up
+// its share of the rows, one word each.
+static bool smem_bitmap(uint64_t words, uint64_t nbt) {
+    return words <= kSmemBitmapWords && words * uint64_t(sm_count()) <= nbt * kBlock;
+}
+
 static int view_or_decompress(const ms_col *c, ms_arena *a, cudaStream_t st, ColView *v) {
     if (c->format != MS_FMT_RLE) return prepare_view(c, a, st, v);
     uint64_t *tmp = arena_take_t<uint64_t>(a, c->count_values + 1);
@@ -770,17 +777,12 @@ extern "C" int ms_gpu_semi_join(const ms_col *l, const ms_col *r, int out_format
     unsigned long long *mm = arena_take_t<unsigned long long>(a, 2);
     int *has_max = arena_take_t<int>(a, 1);
     if (!mm || !has_max) return ms_fail(MS_ERR_NOMEM, "arena exhausted (semi_join)");
-    const unsigned long long init[2] = {~0ull, 0ull};
-    MS_CUDA_TRY(cudaMemcpyAsync(mm, init, 16, cudaMemcpyHostToDevice, st));
-    MS_CUDA_TRY(cudaMemsetAsync(has_max, 0, 4, st));
     const uint64_t nbl = lv.nblocks_total();
+    uint64_t hmm[2] = {0, 0};
     if (nbl) {
-        k_minmax<<<grid_blocks(nbl), 256, 0, st>>>(lv, mm, mm + 1, a->d_err);
-        MS_CUDA_TRY(cudaGetLastError());
+        rc = key_range(lv, mm, hmm, hmm + 1, a, st);
+        if (rc) return rc;
     }
-    unsigned long long hmm[2];
-    MS_CUDA_TRY(cudaMemcpyAsync(hmm, mm, 16, cudaMemcpyDeviceToHost, st));
-    MS_CUDA_TRY(cudaStreamSynchronize(st));
     KeySet s{};
     const uint64_t nl = l->count_values;
     const bool bitmap = nl > 0 && (hmm[1] - hmm[0]) < (uint64_t(1) << 27);
@@ -810,6 +812,7 @@ extern "C" int ms_gpu_semi_join(const ms_col *l, const ms_col *r, int out_format
         MS_CUDA_TRY(cudaMemsetAsync(slots, 0xFF, 8 * cap, st));
         s.slots = slots;
         s.mask = cap - 1;
+        MS_CUDA_TRY(cudaMemsetAsync(has_max, 0, 4, st));
         k_build_set<<<grid_blocks(nbl), 256, 0, st>>>(lv, nullptr, 0, slots, s.mask, has_max, a->d_err);
         MS_CUDA_TRY(cudaGetLastError());
         int hm = 0;
@@ -817,18 +820,22 @@ extern "C" int ms_gpu_semi_join(const ms_col *l, const ms_col *r, int out_format
         MS_CUDA_TRY(cudaStreamSynchronize(st));
         s.has_max = hm;
     }
-    const bool smem = s.bits && (s.span + 31) / 32 <= kSmemBitmapWords;
-    const size_t shm = smem ? 4 * ((s.span + 31) / 32) : 0;
-    if (smem && shm > 48 * 1024)
-        MS_CUDA_TRY(cudaFuncSetAttribute(k_probe<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
+    const uint64_t words = (s.span + 31) / 32;
     const uint64_t nbt = rv.nblocks_total();
-    auto launch = [&](uint32_t *bc, const uint64_t *bo, uint64_t *pos, unsigned long long *scal) {
+    const bool smem = s.bits && smem_bitmap(words, nbt);
+    if (smem)
+        MS_CUDA_TRY(cudaFuncSetAttribute(k_probe_bits<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(4 * words)));
+    auto pass1 = [&](const MaskRun &run, uint32_t *) {
         if (smem)
-            k_probe<true><<<grid_blocks(nbt), 256, shm, st>>>(rv, s, bc, bo, pos, scal, a->d_err);
+            k_probe_bits<true><<<mask_grid(run.nblk, kProbeWarps, 1), 32 * kProbeWarps, 4 * words, st>>>(rv, s, run,
+                                                                                                    a->d_err);
         else
-            k_probe<false><<<grid_blocks(nbt), 256, 0, st>>>(rv, s, bc, bo, pos, scal, a->d_err);
+            k_probe_bits<false><<<mask_grid(run.nblk, 8, 3), 256, 0, st>>>(rv, s, run, a->d_err);
     };
-    return positions_two_pass(nbt, launch, out_format, out_bw, out, a, st);
+    uint64_t *pos, cnt, nscal;
+    rc = rows_by_mask<false, uint32_t>(rv, pass1, &pos, nullptr, &cnt, &nscal, a, st);
+    if (rc) return rc;
+    return write_values(pos, cnt - nscal, nscal, out_format, out_bw, out, a, st);
 }
 
 extern "C" int ms_gpu_intersect_sorted(const ms_col *l, const ms_col *r, int out_format, unsigned out_bw, ms_col *out,
@@ -1036,24 +1043,24 @@ extern "C" int ms_gpu_natural_join(const ms_col *l, const ms_col *r, int out_l_f
     if (rc) return rc;
     unsigned long long *mm = arena_take_t<unsigned long long>(a, 3);
     if (!mm) return ms_fail(MS_ERR_NOMEM, "arena exhausted (natural_join)");
-    const unsigned long long init[3] = {~0ull, 0ull, ~0ull};
-    MS_CUDA_TRY(cudaMemcpyAsync(mm, init, 24, cudaMemcpyHostToDevice, st));
     const uint64_t nbl = lv.nblocks_total(), nl = l->count_values;
+    uint64_t hmm[2] = {0, 0};
     if (nbl) {
-        k_minmax<<<grid_blocks(nbl), 256, 0, st>>>(lv, mm, mm + 1, a->d_err);
-        MS_CUDA_TRY(cudaGetLastError());
+        rc = key_range(lv, mm, hmm, hmm + 1, a, st);
+        if (rc) return rc;
     }
-    unsigned long long hmm[2];
-    MS_CUDA_TRY(cudaMemcpyAsync(hmm, mm, 16, cudaMemcpyDeviceToHost, st));
-    MS_CUDA_TRY(cudaStreamSynchronize(st));
+    MS_CUDA_TRY(cudaMemsetAsync(mm + 2, 0xFF, 8, st));
     KeyMap m{};
     m.max_pos = mm + 2;
-    if (nl && hmm[1] - hmm[0] < (uint64_t(1) << 24)) {
+    if (nl && nl < 0xFFFFFFFFull && hmm[1] - hmm[0] < (uint64_t(1) << 24)) {
         m.lo = hmm[0];
         m.span = hmm[1] - hmm[0] + 1;
-        m.dense = arena_take_t<unsigned long long>(a, m.span);
-        if (!m.dense) return ms_fail(MS_ERR_NOMEM, "arena exhausted (natural_join array)");
-        MS_CUDA_TRY(cudaMemsetAsync(m.dense, 0xFF, 8 * m.span, st));
+        const uint64_t words = (m.span + 31) / 32;
+        m.dense = arena_take_t<uint32_t>(a, m.span);
+        m.bits = arena_take_t<uint32_t>(a, words);
+        if (!m.dense || !m.bits) return ms_fail(MS_ERR_NOMEM, "arena exhausted (natural_join array)");
+        MS_CUDA_TRY(cudaMemsetAsync(m.dense, 0xFF, 4 * m.span, st));
+        MS_CUDA_TRY(cudaMemsetAsync(m.bits, 0, 4 * words, st));
     } else {
         uint64_t cap = 16;
         while (cap < 2 * nl) cap <<= 1;
@@ -1068,36 +1075,27 @@ extern "C" int ms_gpu_natural_join(const ms_col *l, const ms_col *r, int out_l_f
         k_build_map<<<grid_blocks(nbl), 256, 0, st>>>(lv, m, a->d_err);
         MS_CUDA_TRY(cudaGetLastError());
     }
-    // two passes over the probe side: counts, scan, pairs
-    const uint64_t nbt = rv.nblocks_total();
-    uint32_t *bc = arena_take_t<uint32_t>(a, nbt + 1);
-    uint64_t *bo = arena_take_t<uint64_t>(a, nbt + 1);
-    uint64_t *tot = arena_take_t<uint64_t>(a, 2);
-    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(nbt, 1));
-    if (!bc || !bo || !tot || !scr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (natural_join)");
-    MS_CUDA_TRY(cudaMemsetAsync(tot, 0, 16, st));
-    if (nbt) {
-        k_probe_map<<<grid_blocks(nbt), 256, 0, st>>>(rv, m, bc, nullptr, nullptr, nullptr, nullptr, a->d_err);
-        MS_CUDA_TRY(cudaGetLastError());
-        MS_CUDA_TRY((scan_exclusive<uint32_t, 1>(bc, nbt, bo, tot, scr, st)));
-    }
-    uint64_t total = 0;
-    MS_CUDA_TRY(cudaMemcpyAsync(&total, tot, 8, cudaMemcpyDeviceToHost, st));
-    MS_CUDA_TRY(cudaStreamSynchronize(st));
-    uint64_t *pr = arena_take_t<uint64_t>(a, total + 1);
-    uint64_t *pl = arena_take_t<uint64_t>(a, total + 1);
-    if (!pr || !pl) return ms_fail(MS_ERR_NOMEM, "arena exhausted (natural_join output)");
-    if (total) {
-        k_probe_map<<<grid_blocks(nbt), 256, 0, st>>>(rv, m, bc, bo, pr, pl, (unsigned long long *)(tot + 1),
-                                                      a->d_err);
-        MS_CUDA_TRY(cudaGetLastError());
-    }
-    uint64_t scal = 0;
-    MS_CUDA_TRY(cudaMemcpyAsync(&scal, tot + 1, 8, cudaMemcpyDeviceToHost, st));
-    rc = read_err(a, st);
+    const uint64_t words = (m.span + 31) / 32;
+    const bool smem = m.dense && smem_bitmap(words, rv.nblocks_total());
+    uint64_t *pr, *pl, total, scal;
+    // build positions of 32 bits unless the build side is longer
+    auto join = [&](auto pos_type) -> int {
+        using V = decltype(pos_type);
+        if (smem)
+            MS_CUDA_TRY(cudaFuncSetAttribute(k_probe_map_bits<true, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             int(4 * words)));
+        auto pass1 = [&](const MaskRun &run, V *side) {
+            if (smem)
+                k_probe_map_bits<true, V><<<mask_grid(run.nblk, kProbeWarps, 1), 32 * kProbeWarps, 4 * words, st>>>(
+                    rv, m, run, side, a->d_err);
+            else
+                k_probe_map_bits<false, V><<<mask_grid(run.nblk, 8, 3), 256, 0, st>>>(rv, m, run, side, a->d_err);
+        };
+        return rows_by_mask<true, V>(rv, pass1, &pr, &pl, &total, &scal, a, st);
+    };
+    rc = nl < 0xFFFFFFFFull ? join(uint32_t(0)) : join(uint64_t(0));
     if (rc) return rc;
     rc = write_values(pl, total - scal, scal, out_l_format, out_l_bw, out_l, a, st);
     if (rc) return rc;
     return write_values(pr, total - scal, scal, out_r_format, out_r_bw, out_r, a, st);
 }
-

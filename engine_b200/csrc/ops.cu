@@ -8,6 +8,7 @@
 #include <mutex>
 
 #include "internal.h"
+#include "positions.cuh"
 #include "scan.cuh"
 
 namespace ms {
@@ -105,6 +106,40 @@ __global__ void __launch_bounds__(256) k_select_write(ColView x, ColView y, int 
     if (!ok) atomicOr(err, kErrCorrupt);
 }
 
+// Pass 1 of select: hit bits of every row.  Blocks of the compressed part
+// compare inside the bit-width switch on 32-bit fields (for_f: a threshold on
+// the offsets from the block's reference); delta_f, the uncompressed rest and
+// rows compared unsigned decode to 64-bit values first.
+__global__ void __launch_bounds__(256, 4) k_select_bits(ColView x, int cmp, uint64_t val, Pred pred, MaskRun r,
+                                                       unsigned *err) {
+    bool bad = false;
+    const bool fast = x.fmt == MS_FMT_STATIC_VBP || x.fmt == MS_FMT_DYNAMIC_VBP || x.fmt == MS_FMT_FOR_DVBP;
+    mask_pass(r, [&](uint64_t b, unsigned l, unsigned q) -> unsigned {
+        if (fast && b < x.nb() && (b + 1) * kBlock <= x.sfrom) {
+            uint64_t off;
+            unsigned bw;
+            if (x.fmt == MS_FMT_STATIC_VBP) {
+                bw = x.bw;
+                off = b * 64ull * bw;
+            } else {
+                const uint64_t e = __ldg(x.index + b);
+                off = idx_off(e);
+                bw = idx_bw(e);
+            }
+            const uint64_t *blk = reinterpret_cast<const uint64_t *>(x.data + off);
+            Pred p = pred;
+            if (x.fmt != MS_FMT_FOR_DVBP ||
+                (bw <= 32 && rel_pred(__ldg(x.aux + (b >> 1)), uint64_t(1) << bw, val, cmp, p)))
+                return mask_block_rt(bw, blk, l, q, p, bad);
+        }
+        uint64_t v[16];
+        unsigned valid;
+        bad |= !decode_block(x, b, l, q, v, valid);
+        return select_mask(x, b, l, q, v, valid, cmp, val);
+    });
+    if (bad) atomicOr(err, kErrCorrupt);
+}
+
 // rle input: per run (value, length).
 __global__ void k_rle_sps(const uint64_t *__restrict__ pairs, uint64_t runs, bool pred, int cmp, uint64_t val,
                           unsigned long long *__restrict__ d_sum, unsigned long long *__restrict__ d_cnt) {
@@ -170,9 +205,9 @@ static unsigned grid_for_blocks(uint64_t nbt) {
     return (unsigned)maxu(1, minu((nbt + 7) / 8, persistent_grid(256, 8)));
 }
 
-// Pass 1 + scan + pass 2: uncompressed positions (and values of y) into
-// arena arrays; returns counts.
-static int select_positions(const ColView &x, const ColView *y, int cmp, uint64_t val, ms_arena *a, cudaStream_t st,
+// Pass 1 + scan + pass 2: uncompressed positions and values of y into arena
+// arrays; returns counts.
+static int select_positions(const ColView &x, const ColView &y, int cmp, uint64_t val, ms_arena *a, cudaStream_t st,
                             uint64_t **d_pos, uint64_t **d_vals, uint64_t *count, uint64_t *n_scalar) {
     const uint64_t nbt = x.nblocks_total();
     uint32_t *bc = arena_take_t<uint32_t>(a, nbt + 1);
@@ -191,16 +226,12 @@ static int select_positions(const ColView &x, const ColView *y, int cmp, uint64_
     MS_CUDA_TRY(cudaMemcpyAsync(&total, tot, 8, cudaMemcpyDeviceToHost, st));
     MS_CUDA_TRY(cudaStreamSynchronize(st));
     uint64_t *pos = arena_take_t<uint64_t>(a, total + 1);
-    uint64_t *vals = y ? arena_take_t<uint64_t>(a, total + 1) : nullptr;
-    if (!pos || (y && !vals)) return ms_fail(MS_ERR_NOMEM, "arena exhausted (select output)");
+    uint64_t *vals = arena_take_t<uint64_t>(a, total + 1);
+    if (!pos || !vals) return ms_fail(MS_ERR_NOMEM, "arena exhausted (select output)");
     MS_CUDA_TRY(cudaMemsetAsync(tot + 1, 0, 8, st));
     if (total) {
-        if (y)
-            k_select_write<true><<<grid, 256, 0, st>>>(x, *y, cmp, val, bo, pos, vals,
-                                                      (unsigned long long *)(tot + 1), a->d_err);
-        else
-            k_select_write<false><<<grid, 256, 0, st>>>(x, x, cmp, val, bo, pos, nullptr,
-                                                       (unsigned long long *)(tot + 1), a->d_err);
+        k_select_write<true><<<grid, 256, 0, st>>>(x, y, cmp, val, bo, pos, vals, (unsigned long long *)(tot + 1),
+                                                  a->d_err);
         MS_CUDA_TRY(cudaGetLastError());
     }
     uint64_t scal = 0;
@@ -208,7 +239,7 @@ static int select_positions(const ColView &x, const ColView *y, int cmp, uint64_
     int rc = read_err(a, st);
     if (rc) return rc;
     *d_pos = pos;
-    if (d_vals) *d_vals = vals;
+    *d_vals = vals;
     *count = total;
     *n_scalar = scal;
     return MS_OK;
@@ -304,7 +335,11 @@ extern "C" int ms_gpu_select(int cmp, uint64_t val, const ms_col *in, int out_fo
     // whole column, and all hits are written as remainder rows
     if (all_unsigned) x.sfrom = 0;
     uint64_t *pos, cnt, nscal;
-    rc = select_positions(x, nullptr, cmp, val, a, st, &pos, nullptr, &cnt, &nscal);
+    const Pred pred = make_pred(cmp, val);
+    auto pass1 = [&](const MaskRun &r, uint32_t *) {
+        k_select_bits<<<mask_grid(r.nblk, 8, 4), 256, 0, st>>>(x, cmp, val, pred, r, a->d_err);
+    };
+    rc = rows_by_mask<false, uint32_t>(x, pass1, &pos, nullptr, &cnt, &nscal, a, st);
     if (rc) return rc;
     return write_values(pos, cnt - nscal, nscal, out_format, out_bw, out, a, st);
 }
@@ -358,7 +393,7 @@ extern "C" int ms_gpu_select_project_sum(const ms_col *xc, int cmp, uint64_t c, 
     if (rc) return rc;
     if (d_pos || d_vals) {
         uint64_t *pos, *vals, cnt, nscal;
-        rc = select_positions(x, &y, cmp, c, a, st, &pos, &vals, &cnt, &nscal);
+        rc = select_positions(x, y, cmp, c, a, st, &pos, &vals, &cnt, &nscal);
         if (rc) return rc;
         if (d_pos && cnt) MS_CUDA_TRY(cudaMemcpyAsync(d_pos, pos, 8 * cnt, cudaMemcpyDeviceToDevice, st));
         if (d_vals && cnt) MS_CUDA_TRY(cudaMemcpyAsync(d_vals, vals, 8 * cnt, cudaMemcpyDeviceToDevice, st));

@@ -21,6 +21,7 @@
 
 #include "fastpath.cuh"
 #include "internal.h"
+#include "positions.cuh"
 #include "scan.cuh"
 #include "stream.cuh"
 #include "tma.cuh"
@@ -488,27 +489,6 @@ __global__ void k_q3_bits(ColView l, uint64_t lo, uint32_t *bits, unsigned *err)
     if (!ok) atomicOr(err, kErrCorrupt);
 }
 
-__global__ void k_minmax_q(ColView c, unsigned long long *mn, unsigned long long *mx, unsigned *err) {
-    const unsigned lane = threadIdx.x & 31u, l = lane & 7u, q = lane >> 3;
-    uint64_t lo = ~uint64_t(0), hi = 0;
-    bool ok = true;
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < c.nblocks_total();
-         b += uint64_t(gridDim.x) * blockDim.x / 32) {
-        uint64_t v[16];
-        unsigned valid;
-        ok &= decode_block(c, b, l, q, v, valid);
-#pragma unroll
-        for (int k = 0; k < 16; k++)
-            if ((valid >> k) & 1u) {
-                lo = minu(lo, v[k]);
-                hi = maxu(hi, v[k]);
-            }
-    }
-    if (!ok) atomicOr(err, kErrCorrupt);
-    atomicMin(mn, (unsigned long long)lo);
-    atomicMax(mx, (unsigned long long)hi);
-}
-
 // Extent of every group: its first row's position in P, i.e. the hits in
 // earlier blocks (scan of the per-block counts) plus the row's rank among the
 // hits of its own block, which one warp per group recomputes by decoding that
@@ -712,16 +692,9 @@ extern "C" int ms_gpu_query3(const ms_col *filter, int cmp, uint64_t c, const ms
     // build side bitmap
     unsigned long long *mm = arena_take_t<unsigned long long>(a, 2);
     if (!mm) return ms_fail(MS_ERR_NOMEM, "arena exhausted (query3)");
-    const unsigned long long init[2] = {~0ull, 0ull};
-    MS_CUDA_TRY(cudaMemcpyAsync(mm, init, 16, cudaMemcpyHostToDevice, st));
     const unsigned grid = unsigned(maxu(1, minu((lv.nblocks_total() + 7) / 8, persistent_grid(256, 8))));
-    if (lv.n) {
-        k_minmax_q<<<grid, 256, 0, st>>>(lv, mm, mm + 1, a->d_err);
-        MS_CUDA_TRY(cudaGetLastError());
-    }
-    unsigned long long hmm[2];
-    MS_CUDA_TRY(cudaMemcpyAsync(hmm, mm, 16, cudaMemcpyDeviceToHost, st));
-    MS_CUDA_TRY(cudaStreamSynchronize(st));
+    uint64_t hmm[2] = {0, 0};
+    if (lv.n && (rc = key_range(lv, mm, hmm, hmm + 1, a, st))) return rc;
     uint64_t lo = 0, span = 0;
     if (lv.n) {
         lo = hmm[0];

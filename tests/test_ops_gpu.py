@@ -179,3 +179,41 @@ def test_threshold_path_every_width(ms, arena, orc, bw):
     finally:
         ms.set_tuning(**old)
 
+
+
+@pytest.mark.parametrize("code,bw", IN_FORMATS)
+@pytest.mark.parametrize("n", [1, 31, 33, 8191, 8192, 8193, 3 * 8192 + 512, 90_007])
+@pytest.mark.parametrize("cut", [0, 40, 512, 600, 4096])
+def test_select_tile_edges_and_densities(ms, arena, orc, code, bw, n, cut):
+    """Positions expanded from bits: words with few and with many hits, steps
+    of 8192 rows cut off at every place, no hits and all hits."""
+    v = _data(orc, code, n, seed=n + cut)
+    c = _col(ms, arena, orc, v, code, bw)
+    sf = orc.scalar_from(code, bw, c.meta())
+    assert np.array_equal(ms.select(O.CMP_LT, c, cut).to_numpy(), orc.select(O.CMP_LT, cut, v, sf))
+
+
+@pytest.mark.parametrize("cut", [0, 41, 2048])
+def test_select_and_joins_in_a_full_arena(ms, orc, cut):
+    """With no room for the bits of all rows at once the operators work in
+    segments; the positions themselves are all that has to fit."""
+    n = 300_007
+    v = orc.uniform_bits(5, 12, n)
+    keys = np.arange(cut, dtype=np.uint64)
+    pos = orc.select(O.CMP_LT, cut, v, n - n % 8)
+    spare = 12 * (n // 512 + 1) + (16 << 10)
+    for op in ("select", "semi_join", "natural_join"):
+        a = ms.Arena(8 * n + 8 * len(pos) * (2 if op == "natural_join" else 1) + 12 * len(keys) + spare)
+        try:
+            col = ms.Column.from_numpy(v, a)
+            if op == "select":
+                got = ms.select(O.CMP_LT, col, cut).to_numpy()
+            elif op == "semi_join":
+                got = ms.semi_join(ms.Column.from_numpy(keys, a), col).to_numpy()
+            else:
+                l, r = ms.natural_join(ms.Column.from_numpy(keys, a), col)
+                got = r.to_numpy()
+                assert np.array_equal(l.to_numpy(), v[pos.astype(np.int64)])
+            assert np.array_equal(got, pos)
+        finally:
+            a.close()
