@@ -1,22 +1,22 @@
 // codecs.cu -- compression and decompression kernels for every format and
 // the column-level morph (morph.h:81-241).
 //
-// Encoding a dynamic_vbp-family column is size-then-scatter:
-//   1. k_analyze: one warp per 512-value block computes the block's bit width
-//      (OR-reduce, dynamic_vbp.h:124-158) after the cascade transform
-//      (delta: x[i]-x[i-8], delta.h:107-156; for: minus the block minimum,
-//      for.h:121-161);
-//   2. an exclusive scan of the bit widths gives every block's byte offset:
-//      64 * (headers before the block) + 64 * (sum of earlier widths);
-//   3. k_pack: one thread per lane stream (8 per block) packs the block at
-//      its offset and records the block index entry; k_headers writes the
-//      page headers (bit-width bytes / 0xFF, FOR reference words).
+// Encoding a dynamic_vbp-family column is one pass in rounds (rounds.cuh):
+// a tile of 12 blocks is staged in shared memory, its block widths found
+// (OR-reduce, dynamic_vbp.h:124-158) after the cascade transform (delta:
+// x[i]-x[i-8], delta.h:107-156; for: minus the block minimum,
+// for.h:121-161), and once the widths before it are known the blocks are
+// packed in place and copied to their offsets -- 64 * (headers before the
+// block) + 64 * (sum of earlier widths) -- with page headers (bit-width bytes /
+// 0xFF, FOR reference words) and block index entries.
 // The same encoder writes operator outputs with the write iterator's
 // 2048-value chunking (write_iterator.h:67-306): only the number of blocks
 // per page changes (64 -> 4 for dynamic_vbp, 8 -> 2 for for_f).
 #include <string.h>
 
+#include "fastpath.cuh"
 #include "internal.h"
+#include "rounds.cuh"
 #include "scan.cuh"
 #include "tma.cuh"
 
@@ -25,188 +25,293 @@ namespace {
 
 struct Layout {
     int fmt;
-    unsigned bw;           // static_vbp
-    unsigned dvbp_page;    // blocks per dynamic_vbp page (64 morph, 4 write iterator)
-    unsigned for_page;     // cascade blocks per for_f page (8 morph, 2 write iterator)
+    unsigned bw;          // static_vbp
+    unsigned dvbp_shift;  // log2 of blocks per dynamic_vbp page (6 morph, 2 write iterator)
+    unsigned for_shift;   // log2 of cascade blocks per for_f page (3 morph, 1 write iterator)
 };
 
 // 64-B headers preceding block b's packed data.
-__host__ __device__ inline uint64_t headers_before(const Layout &L, uint64_t b) {
-    switch (L.fmt) {
-    case MS_FMT_DYNAMIC_VBP: return b / L.dvbp_page + 1;
+template <int FMT>
+__device__ __forceinline__ uint64_t headers_before(const Layout &L, uint64_t b) {
+    switch (FMT) {
+    case MS_FMT_DYNAMIC_VBP: return (b >> L.dvbp_shift) + 1;
     case MS_FMT_DELTA_DVBP: return b / 2 + 1;
-    case MS_FMT_FOR_DVBP: return b / (2 * L.for_page) + 1 + b / 2 + 1;
-    default: return 0;
+    default: return (b >> (1 + L.for_shift)) + 1 + b / 2 + 1;
     }
 }
 
-__device__ __forceinline__ uint64_t warp_or(uint64_t x) {
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) x |= __shfl_xor_sync(0xFFFFFFFFu, x, s);
-    return x;
-}
-
-// --- 1. analysis -----------------------------------------------------------
-// dynamic_vbp / delta: one warp per 512-block.
-template <int FMT>
-__global__ void __launch_bounds__(256) k_analyze_blocks(const uint64_t *__restrict__ in, uint64_t nb,
-                                                       uint32_t *__restrict__ bw_out) {
-    const unsigned lane = threadIdx.x & 31u;
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < nb;
-         b += uint64_t(gridDim.x) * blockDim.x / 32) {
-        const uint64_t *blk = in + b * kBlock;
-        uint64_t acc = 1;
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const unsigned r = k * 32 + lane;  // coalesced rows
-            uint64_t x = __ldg(blk + r);
-            if (FMT == MS_FMT_DELTA_DVBP) {
-                const uint64_t row = b * kBlock + r;
-                x -= row >= 8 ? __ldg(in + row - 8) : 0;
-            }
-            acc |= x;
-        }
-        acc = warp_or(acc);
-        if (lane == 0) bw_out[b] = effective_bitwidth(acc);
-    }
-}
-
-// for_f: one warp per 1024-block; reference = AVX-512 TVL minimum (signed
-// per lane, _mm512_min_epi64, then unsigned across lanes; for.h:121-161).
-__global__ void __launch_bounds__(256) k_analyze_for(const uint64_t *__restrict__ in, uint64_t ncb,
-                                                    uint32_t *__restrict__ bw_out, uint64_t *__restrict__ refs) {
-    const unsigned lane = threadIdx.x & 31u;
-    for (uint64_t c = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; c < ncb;
-         c += uint64_t(gridDim.x) * blockDim.x / 32) {
-        const uint64_t *blk = in + c * kCascBlock;
-        // lane & 7 is the TVL lane of every row this thread reads
-        int64_t mn = INT64_MAX;
-        uint64_t x[32];
-#pragma unroll
-        for (int k = 0; k < 32; k++) {
-            x[k] = __ldg(blk + k * 32 + lane);
-            mn = min(mn, (int64_t)x[k]);
-        }
-        mn = min(mn, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (uint64_t)mn, 8));
-        mn = min(mn, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (uint64_t)mn, 16));
-        uint64_t um = (uint64_t)mn;
-        um = min(um, __shfl_xor_sync(0xFFFFFFFFu, um, 1));
-        um = min(um, __shfl_xor_sync(0xFFFFFFFFu, um, 2));
-        um = min(um, __shfl_xor_sync(0xFFFFFFFFu, um, 4));
-        if (um == ~uint64_t(0)) um--;
-        uint64_t o0 = 1, o1 = 1;
-#pragma unroll
-        for (int k = 0; k < 16; k++) o0 |= x[k] - um;
-#pragma unroll
-        for (int k = 16; k < 32; k++) o1 |= x[k] - um;
-        o0 = warp_or(o0);
-        o1 = warp_or(o1);
-        if (lane == 0) {
-            refs[c] = um;
-            bw_out[2 * c] = effective_bitwidth(o0);
-            bw_out[2 * c + 1] = effective_bitwidth(o1);
-        }
-    }
-}
-
-// --- 3. packing -------------------------------------------------------------
+// --- packing: static_vbp ------------------------------------------------------
 // Eight threads per block, one per lane stream; a warp packs four blocks.
-template <int FMT>
-__global__ void __launch_bounds__(256) k_pack(const uint64_t *__restrict__ in, uint64_t nb, Layout L,
-                                             const uint32_t *__restrict__ bws, const uint64_t *__restrict__ prefix,
-                                             const uint64_t *__restrict__ refs, uint8_t *__restrict__ out,
-                                             uint64_t *__restrict__ index, unsigned *err) {
+__global__ void __launch_bounds__(256) k_pack_static(const uint64_t *__restrict__ in, uint64_t nb, unsigned bw,
+                                                    uint8_t *__restrict__ out, unsigned *err) {
     const unsigned l = threadIdx.x & 7u;
     for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 8; b < nb;
          b += uint64_t(gridDim.x) * blockDim.x / 8) {
-        unsigned bw;
-        uint64_t off;
-        if (FMT == MS_FMT_STATIC_VBP) {
-            bw = L.bw;
-            off = b * 64ull * bw;
-        } else {
-            bw = bws[b];
-            off = 64ull * headers_before(L, b) + 64ull * prefix[b];
-            if (l == 0 && index) index[b] = idx_pack(off, bw);
-        }
         const uint64_t *blk = in + b * kBlock;
-        const uint64_t ref = FMT == MS_FMT_FOR_DVBP ? refs[b >> 1] : 0;
-        auto get = [&](unsigned v) -> uint64_t {
-            const unsigned r = v * 8 + l;
-            uint64_t x = __ldg(blk + r);
-            if (FMT == MS_FMT_DELTA_DVBP) {
-                const uint64_t row = b * kBlock + r;
-                x -= row >= 8 ? __ldg(in + row - 8) : 0;
-            } else if (FMT == MS_FMT_FOR_DVBP) {
-                x -= ref;
-            }
-            return x;
-        };
-        if (!vbp_pack_lane_rt(bw, get, reinterpret_cast<uint64_t *>(out + off), l)) atomicOr(err, kErrCorrupt);
+        auto get = [&](unsigned v) -> uint64_t { return __ldg(blk + v * 8 + l); };
+        if (!vbp_pack_lane_rt(bw, get, reinterpret_cast<uint64_t *>(out + b * 64ull * bw), l)) atomicOr(err, kErrCorrupt);
     }
 }
 
-// Page headers.  dynamic_vbp: one thread per header byte.
-__global__ void k_headers_dvbp(uint64_t nb, Layout L, const uint32_t *__restrict__ bws,
-                               const uint64_t *__restrict__ prefix, uint8_t *__restrict__ out) {
-    const uint64_t pages = (nb + L.dvbp_page - 1) / L.dvbp_page;
+// --- dynamic_vbp family: one pass in rounds -----------------------------------
+// Packing: thread (l, h) of a half-warp holds values 32h .. 32h+31 of lane l's
+// stream of a block; they are exactly BW 32-bit words of the packed stream.
+// dst: the block's first byte in shared memory.
+template <unsigned BW>
+__device__ __forceinline__ void pack_half(const uint64_t (&x)[32], uint8_t *dst, unsigned l, unsigned h) {
+    uint32_t w[BW];
+#pragma unroll
+    for (unsigned j = 0; j < BW; j++) w[j] = 0;
+#pragma unroll
+    for (unsigned v = 0; v < 32; v++) {
+        const uint32_t lo = uint32_t(x[v]), hi = uint32_t(x[v] >> 32);
+        const unsigned bit = v * BW, wi = bit >> 5, sh = bit & 31u;
+        w[wi] |= lo << sh;
+        if (BW <= 32) {
+            if (sh + BW > 32) w[wi + 1] |= lo >> (32 - sh);
+        } else {
+            w[wi + 1] |= __funnelshift_l(lo, hi, sh);
+            if (sh + BW > 64) w[wi + 2] |= hi >> (32 - sh);
+        }
+    }
+    uint8_t *o = dst + 8u * l + h * (BW / 2) * 64u;
+    if (BW % 2 == 0) {
+#pragma unroll
+        for (unsigned j = 0; j < BW; j += 2)
+            *reinterpret_cast<uint64_t *>(o + 32u * j) = uint64_t(w[j + (j + 1 < BW ? 1 : 0)]) << 32 | w[j];
+    } else {
+        // the second half starts in the middle of a 64-bit word
+#pragma unroll
+        for (unsigned j = 0; j < BW; j++)
+            *reinterpret_cast<uint32_t *>(o + (h ? ((j + 1) >> 1) * 64u + ((j + 1) & 1u) * 4u
+                                                 : (j >> 1) * 64u + (j & 1u) * 4u)) = w[j];
+    }
+}
+
+__device__ __forceinline__ void pack_half_rt(unsigned bw, const uint64_t (&x)[32], uint8_t *dst, unsigned l, unsigned h) {
+    switch (bw) {
+#define MS_X(B) \
+    case B: pack_half<B>(x, dst, l, h); break;
+        MS_BW_CASES(MS_X)
+#undef MS_X
+    default: break;  // widths come from effective_bitwidth
+    }
+}
+
+constexpr unsigned kEncBlocks = kRdRows / kBlock;  // 12 blocks per tile, two per warp
+// rest rows that the last tile's warps copy themselves
+constexpr uint64_t kEncRest = 4096;
+
+template <int FMT>
+__global__ void __launch_bounds__(kRdThreads, 1)
+    k_encode(const uint64_t *__restrict__ in, uint64_t nb, Layout L, unsigned *words, uint8_t *__restrict__ out,
+             uint64_t *__restrict__ index, uint64_t *__restrict__ refs, uint64_t nrest, uint64_t *__restrict__ d_compr,
+             unsigned *err) {
+    extern __shared__ __align__(128) uint8_t rd_smem[];
+    __shared__ RdShared sh;
+    __shared__ unsigned s_bw[kRdBufs][kEncBlocks];  // by buffer
+    __shared__ uint64_t s_ref[kRdBufs][kEncBlocks / 2];
+    const unsigned tid = threadIdx.x % kRdHalf, w = tid >> 5, lane = tid & 31u;
+    const unsigned l = lane & 7u, h = (lane >> 3) & 1u, half = lane >> 4, j = 2 * w + half;
+    const bool first_half = threadIdx.x < kRdHalf;
+    const uint64_t ntiles = (nb + kEncBlocks - 1) / kEncBlocks;
+    const unsigned rounds = unsigned((ntiles + gridDim.x - 1) / gridDim.x);
+    auto tile_of = [&](unsigned r) { return uint64_t(r) * gridDim.x + blockIdx.x; };
+    auto blocks_of = [&](uint64_t t) { return unsigned(minu(kEncBlocks, nb - t * kEncBlocks)); };
+    auto load = [&](unsigned r) {
+        const uint64_t t = tile_of(r);
+        if (t < ntiles)
+            rd_load(rd_buf(rd_smem, r), sh.full + r % kRdBufs, in, t * kRdRows, blocks_of(t) * kBlock,
+                    FMT == MS_FMT_DELTA_DVBP && t ? 8u : 0u);
+    };
+    rd_init(sh);
+    if (threadIdx.x == 0) {
+        for (unsigned r = 0; r < kRdBufs; r++) load(r);
+    }
+    RdPrefix pre(words, ntiles);
+    for (unsigned r = 0; r <= rounds + 1; r++) {
+        const uint64_t t = tile_of(r);
+        if (first_half && t < ntiles) {
+            const unsigned nblk = blocks_of(t), par = r % kRdBufs;
+            const bool mine = j < nblk;
+            uint8_t *const blk = rd_buf(rd_smem, r) + rd_row(kBlock * j);
+            rd_full(sh, r);
+            // The thread's 32 values.  The two halves read the values of a
+            // pair in opposite order: halves and blocks lie a multiple of 128
+            // bytes apart, so that in the same order all four groups of eight
+            // threads would meet in the same banks.
+            uint64_t x[32], acc = 1;
+            {
+                const uint8_t *const v0 = blk + 8u * (256u * h + l);
+                const uint8_t *const p0 = v0 + 64u * h, *const p1 = v0 + 64u - 64u * h;
+#pragma unroll
+                for (unsigned v = 0; v < 32; v += 2) {
+                    const uint64_t a = mine ? *reinterpret_cast<const uint64_t *>(p0 + 64u * v) : 0;
+                    const uint64_t b = mine ? *reinterpret_cast<const uint64_t *>(p1 + 64u * v) : 0;
+                    x[v] = h ? b : a;
+                    x[v + 1] = h ? a : b;
+                }
+                if (FMT == MS_FMT_DELTA_DVBP) {
+                    const bool none = !mine || (t == 0 && j == 0 && h == 0);  // the column's first rows
+                    const uint64_t prev = none ? 0 : *reinterpret_cast<const uint64_t *>(v0 - 64);
+#pragma unroll
+                    for (int v = 31; v > 0; v--) x[v] -= x[v - 1];
+                    x[0] -= prev;
+                }
+            }
+            if (FMT == MS_FMT_FOR_DVBP) {
+                // the warp's pair is one 1024-block; its reference is the
+                // AVX-512 TVL minimum (signed per lane, _mm512_min_epi64, then
+                // unsigned across lanes; for.h:121-161); l is the TVL lane
+                int64_t mn = INT64_MAX;
+#pragma unroll
+                for (unsigned v = 0; v < 32; v++) mn = min(mn, (int64_t)x[v]);
+                mn = min(mn, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (uint64_t)mn, 8));
+                mn = min(mn, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (uint64_t)mn, 16));
+                uint64_t um = (uint64_t)mn;
+                um = minu(um, __shfl_xor_sync(0xFFFFFFFFu, um, 1));
+                um = minu(um, __shfl_xor_sync(0xFFFFFFFFu, um, 2));
+                um = minu(um, __shfl_xor_sync(0xFFFFFFFFu, um, 4));
+                if (um == ~uint64_t(0)) um--;
+#pragma unroll
+                for (unsigned v = 0; v < 32; v++) x[v] -= um;
+                if (lane == 0 && mine) {
+                    s_ref[par][w] = um;
+                    refs[t * (kEncBlocks / 2) + w] = um;
+                }
+            }
+#pragma unroll
+            for (unsigned v = 0; v < 32; v++) acc |= x[v];
+            // widths of the warp's two blocks
+            const unsigned h0 = __reduce_or_sync(0xFFFFFFFFu, half ? 0u : unsigned(acc >> 32));
+            const unsigned h1 = __reduce_or_sync(0xFFFFFFFFu, half ? unsigned(acc >> 32) : 0u);
+            const unsigned l0 = __reduce_or_sync(0xFFFFFFFFu, half ? 0u : unsigned(acc));
+            const unsigned l1 = __reduce_or_sync(0xFFFFFFFFu, half ? unsigned(acc) : 0u);
+            const unsigned bw = effective_bitwidth(half ? uint64_t(h1) << 32 | l1 : uint64_t(h0) << 32 | l0);
+            if ((lane & 15u) == 0 && mine) s_bw[par][j] = bw;
+            rd_bar(0);  // every value of the tile is in registers
+            if (w == kRdWarps - 1) {
+                const unsigned sum = __reduce_add_sync(0xFFFFFFFFu, lane < nblk ? s_bw[par][lane] : 0u);
+                if (lane == 0) rd_publish(words, t, sum);
+            }
+            if (mine) pack_half_rt(bw, x, blk, l, h);
+        }
+        if (!first_half && r && r <= rounds) pre.request(r - 1, tid);  // read in the next round
+        if (!first_half && r > 1) {
+            // tile r - 2, packed in place, goes to its place, and its buffer
+            // takes tile r + 2
+            const uint64_t tp = tile_of(r - 2);
+            pre.sums(sh, r - 2, tid);
+            if (tp < ntiles) {
+                const unsigned nblk = blocks_of(tp), par = (r - 2) % kRdBufs;
+                const uint8_t *const stage = rd_buf(rd_smem, r - 2) + rd_row(kBlock * j);  // the half-warp's packed block
+                const unsigned bl = lane < nblk ? s_bw[par][lane] : 0u;
+                unsigned ex = bl;  // widths of the tile's blocks before each
+    #pragma unroll
+                for (int d = 1; d < 16; d <<= 1) {
+                    const unsigned o = __shfl_up_sync(0xFFFFFFFFu, ex, d);
+                    if (int(lane) >= d) ex += o;
+                }
+                const unsigned before = __shfl_sync(0xFFFFFFFFu, ex - bl, j), bwp = __shfl_sync(0xFFFFFFFFu, bl, j);
+                const unsigned bw1 = __shfl_sync(0xFFFFFFFFu, bl, 2 * w + 1);  // 0 when the pair has one block
+                const bool mine = j < nblk;
+                const uint64_t b = tp * kEncBlocks + j;
+                const uint64_t off = 64ull * headers_before<FMT>(L, b) + 64ull * (pre.base + pre.lower + before);
+                if (mine) {
+                    // 16 bytes per thread and step, four steps in flight
+                    const uint4 *from = reinterpret_cast<const uint4 *>(stage);
+                    uint4 *to = reinterpret_cast<uint4 *>(out + off);
+                    for (unsigned i0 = lane & 15u; i0 < 4u * bwp; i0 += 64) {
+                        uint4 q[4];
+    #pragma unroll
+                        for (unsigned i = 0; i < 4; i++)
+                            if (i0 + 16u * i < 4u * bwp) q[i] = from[i0 + 16u * i];
+    #pragma unroll
+                        for (unsigned i = 0; i < 4; i++)
+                            if (i0 + 16u * i < 4u * bwp) to[i0 + 16u * i] = q[i];
+                    }
+                    if ((lane & 15u) == 0) index[b] = idx_pack(off, bwp);
+                }
+                if (FMT == MS_FMT_DYNAMIC_VBP) {
+                    // pages of at most four blocks: the header is written with
+                    // the page's first block (larger pages: k_headers_dvbp)
+                    const unsigned page = 1u << L.dvbp_shift;
+                    if (page <= 4 && mine && (j & (page - 1)) == 0 && (lane & 15u) < 8) {
+                        uint64_t word = ~uint64_t(0);
+                        if ((lane & 7u) == 0)
+                            for (unsigned i = 0; i < page && j + i < nblk; i++)
+                                word = (word & ~(0xFFull << (8 * i))) | uint64_t(s_bw[par][j + i]) << (8 * i);
+                        reinterpret_cast<uint64_t *>(out + off - 64)[lane & 7u] = word;
+                    }
+                } else if (mine && lane < 8) {
+                    // inner dynamic_vbp header of the 1024-block: two widths,
+                    // 62 x 0xFF
+                    uint64_t word = ~uint64_t(0);
+                    if (lane == 0) word = (~uint64_t(0) << 16) | uint64_t(bwp) | uint64_t(bw1) << 8;
+                    reinterpret_cast<uint64_t *>(out + off - 64)[lane] = word;
+                    const unsigned page = 1u << L.for_shift;
+                    if (FMT == MS_FMT_FOR_DVBP && page <= 2 && (w & (page - 1)) == 0) {
+                        // page header: references, end marker, zeros (larger
+                        // pages: k_headers_for)
+                        const unsigned nbp = min(page, nblk / 2 - w);
+                        reinterpret_cast<uint64_t *>(out + off - 128)[lane] =
+                            lane < nbp ? s_ref[par][w + lane] : lane == nbp ? ~uint64_t(0) : 0;
+                    }
+                }
+                if (tp == ntiles - 1) {
+                    // the column's end: the compressed size, a short rest behind it
+                    const unsigned in_tile = __reduce_add_sync(0xFFFFFFFFu, bl);
+                    const uint64_t compr = 64ull * headers_before<FMT>(L, nb - 1) + 64ull * (pre.base + pre.lower + in_tile);
+                    if (tid == 0) *d_compr = compr;
+                    if (nrest <= kEncRest) {
+                        uint64_t *dst = reinterpret_cast<uint64_t *>(out + rest_offset(FMT, 0, compr));
+                        for (unsigned i = tid; i < nrest; i += kRdHalf) dst[i] = __ldg(in + nb * kBlock + i);
+                    }
+                }
+            }
+            pre.next();
+            fence_async_smem();  // the buffer's last accesses, before a bulk copy overwrites it
+            rd_bar(1);
+            if (tid == 0) load(r + 2);
+        }
+        if (first_half) fence_async_smem();
+        else pre.turn();
+        __syncthreads();
+    }
+    if (sh.fail && threadIdx.x == 0) atomicOr(err, kErrTimeout);
+}
+
+// Headers of dynamic_vbp pages longer than a tile: one thread per header byte.
+__global__ void k_headers_dvbp(uint64_t nb, unsigned page, const uint64_t *__restrict__ index,
+                               uint8_t *__restrict__ out) {
+    const uint64_t pages = (nb + page - 1) / page;
     for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < pages * kPageBlocks;
          t += uint64_t(gridDim.x) * blockDim.x) {
-        const uint64_t p = t / kPageBlocks, j = t % kPageBlocks, b0 = p * L.dvbp_page;
-        const uint64_t start = 64ull * headers_before(L, b0) + 64ull * prefix[b0] - 64;
-        const uint64_t b = b0 + j;
-        out[start + j] = (j < L.dvbp_page && b < nb) ? uint8_t(bws[b]) : uint8_t(kNoBlock);
+        const uint64_t p = t / kPageBlocks, j = t % kPageBlocks, b = p * page + j;
+        out[idx_off(index[p * page]) - 64 + j] = (j < page && b < nb) ? uint8_t(idx_bw(index[b])) : uint8_t(kNoBlock);
     }
 }
 
-// delta / for: inner dynamic_vbp header of each 1024-block (2 widths + 62 x
-// 0xFF) and, for for_f, the page header of reference words.
-template <int FMT>
-__global__ void k_headers_casc(uint64_t nb, Layout L, const uint32_t *__restrict__ bws,
-                               const uint64_t *__restrict__ prefix, const uint64_t *__restrict__ refs,
-                               uint8_t *__restrict__ out) {
-    const uint64_t ncb = nb / 2;
-    for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < ncb * 8;
-         t += uint64_t(gridDim.x) * blockDim.x) {
-        const uint64_t c = t / 8, w = t % 8;
-        const uint64_t start = 64ull * headers_before(L, 2 * c) + 64ull * prefix[2 * c] - 64;
-        uint64_t word = ~uint64_t(0);
-        if (w == 0) word = (~uint64_t(0) << 16) | uint64_t(bws[2 * c] & 0xFF) | (uint64_t(bws[2 * c + 1] & 0xFF) << 8);
-        reinterpret_cast<uint64_t *>(out + start)[w] = word;
-        if (FMT == MS_FMT_FOR_DVBP && c % L.for_page == 0) {
-            const uint64_t fstart = start - 64;
-            const uint64_t nbp = minu(L.for_page, ncb - c);
-            uint64_t fw;
-            if (w < nbp) fw = refs[c + w];
-            else if (w == nbp) fw = ~uint64_t(0);
-            else fw = 0;
-            reinterpret_cast<uint64_t *>(out + fstart)[w] = fw;
-        }
+// Headers of for_f pages longer than a tile: references, end marker, zeros.
+__global__ void k_headers_for(uint64_t ncb, unsigned page, const uint64_t *__restrict__ index,
+                              const uint64_t *__restrict__ refs, uint8_t *__restrict__ out) {
+    const uint64_t pages = (ncb + page - 1) / page;
+    for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < pages * 8; t += uint64_t(gridDim.x) * blockDim.x) {
+        const uint64_t c = t / 8 * page, w = t % 8, nbp = minu(page, ncb - c);
+        reinterpret_cast<uint64_t *>(out + idx_off(index[2 * c]) - 128)[w] =
+            w < nbp ? refs[c + w] : w == nbp ? ~uint64_t(0) : 0;
     }
 }
 
 // Uncompressed rest: copied behind the gap (morph.h:186-189,
-// write_iterator.h:157-170).  The compressed size is read on the device.
+// write_iterator.h:157-170).  A compressed size known on the device only is
+// read there.
 __global__ void k_copy_rest(const uint64_t *__restrict__ in, uint64_t nrest, int fmt, unsigned bw,
-                            const uint64_t *__restrict__ d_compr, uint8_t *__restrict__ out) {
-    const uint64_t ro = rest_offset(fmt, bw, *d_compr);
+                            const uint64_t *__restrict__ d_compr, uint64_t compr, uint8_t *__restrict__ out) {
+    const uint64_t ro = rest_offset(fmt, bw, d_compr ? *d_compr : compr);
     uint64_t *dst = reinterpret_cast<uint64_t *>(out + ro);
     for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nrest; i += uint64_t(gridDim.x) * blockDim.x)
         dst[i] = in[i];
-}
-
-__global__ void k_finish_sizes(uint64_t nb, Layout L, const uint32_t *__restrict__ bws,
-                               const uint64_t *__restrict__ prefix, uint64_t *__restrict__ d_compr) {
-    if (threadIdx.x || blockIdx.x) return;
-    if (nb == 0) {
-        *d_compr = 0;
-        return;
-    }
-    if (L.fmt == MS_FMT_STATIC_VBP) {
-        *d_compr = nb * 64ull * L.bw;
-        return;
-    }
-    *d_compr = 64ull * headers_before(L, nb - 1) + 64ull * prefix[nb - 1] + 64ull * bws[nb - 1];
 }
 
 // --- decompression ------------------------------------------------------------
@@ -952,65 +1057,72 @@ static int decode_rle(const ms_col *in, uint64_t *d_out, ms_arena *a, cudaStream
     return MS_OK;
 }
 
+// Launch of a rounds kernel: one CTA per SM at most, all resident.
+template <class... P, class... A>
+static int launch_rounds(void (*kern)(P...), uint64_t ntiles, cudaStream_t st, A... args) {
+    constexpr size_t smem = kRdSmem;
+    MS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    lc.gridDim = dim3(unsigned(minu(ntiles, uint64_t(sm_count()))));
+    lc.blockDim = dim3(kRdThreads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    MS_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, P(args)...));
+    return MS_OK;
+}
+
 // Shared encoder: `ncompr` rows (a block multiple) go to the compressed part
 // with page layout L, rows [ncompr, n) to the uncompressed rest.
 static int encode(const uint64_t *d_in, uint64_t n, uint64_t ncompr, Layout L, ms_col *out, ms_arena *a,
                   cudaStream_t st) {
     const int fmt = L.fmt;
-    const uint64_t nb = ncompr / kBlock;
+    const uint64_t nb = ncompr / kBlock, nrest = n - ncompr;
     const uint64_t cap = ms_size_max_byte_any_len(fmt, L.bw, n);
     uint8_t *data = arena_take_t<uint8_t>(a, cap);
-    uint64_t *d_compr = arena_take_t<uint64_t>(a, 1);
-    uint64_t *index = nullptr, *aux = nullptr;
-    uint32_t *bws = nullptr;
-    uint64_t *prefix = nullptr, *tot = nullptr, *scr = nullptr, *refs = nullptr;
-    if (!data || !d_compr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (encode)");
+    if (!data) return ms_fail(MS_ERR_NOMEM, "arena exhausted (encode)");
+    uint64_t *index = nullptr, *refs = nullptr, *d_compr = nullptr;
     const unsigned grid = persistent_grid(256, 8);
-    if (fmt != MS_FMT_STATIC_VBP && nb) {
-        index = arena_take_t<uint64_t>(a, nb + 1);
-        bws = arena_take_t<uint32_t>(a, nb + 1);
-        prefix = arena_take_t<uint64_t>(a, nb + 1);
-        tot = arena_take_t<uint64_t>(a, 1);
-        scr = arena_take_t<uint64_t>(a, scan_scratch_words(nb, 1));
-        if (fmt == MS_FMT_FOR_DVBP) aux = refs = arena_take_t<uint64_t>(a, nb / 2 + 1);
-        if (!index || !bws || !prefix || !tot || !scr || (fmt == MS_FMT_FOR_DVBP && !refs))
-            return ms_fail(MS_ERR_NOMEM, "arena exhausted (encode scratch)");
-        if (fmt == MS_FMT_DYNAMIC_VBP) k_analyze_blocks<MS_FMT_DYNAMIC_VBP><<<grid, 256, 0, st>>>(d_in, nb, bws);
-        else if (fmt == MS_FMT_DELTA_DVBP) k_analyze_blocks<MS_FMT_DELTA_DVBP><<<grid, 256, 0, st>>>(d_in, nb, bws);
-        else k_analyze_for<<<grid, 256, 0, st>>>(d_in, nb / 2, bws, refs);
-        MS_CUDA_TRY(cudaGetLastError());
-        MS_CUDA_TRY((scan_exclusive<uint32_t, 1>(bws, nb, prefix, tot, scr, st)));
-    }
-    if (nb) {
-        switch (fmt) {
-        case MS_FMT_STATIC_VBP:
-            k_pack<MS_FMT_STATIC_VBP><<<grid, 256, 0, st>>>(d_in, nb, L, bws, prefix, refs, data, index, a->d_err);
-            break;
-        case MS_FMT_DYNAMIC_VBP:
-            k_pack<MS_FMT_DYNAMIC_VBP><<<grid, 256, 0, st>>>(d_in, nb, L, bws, prefix, refs, data, index, a->d_err);
-            k_headers_dvbp<<<grid, 256, 0, st>>>(nb, L, bws, prefix, data);
-            break;
-        case MS_FMT_DELTA_DVBP:
-            k_pack<MS_FMT_DELTA_DVBP><<<grid, 256, 0, st>>>(d_in, nb, L, bws, prefix, refs, data, index, a->d_err);
-            k_headers_casc<MS_FMT_DELTA_DVBP><<<grid, 256, 0, st>>>(nb, L, bws, prefix, refs, data);
-            break;
-        case MS_FMT_FOR_DVBP:
-            k_pack<MS_FMT_FOR_DVBP><<<grid, 256, 0, st>>>(d_in, nb, L, bws, prefix, refs, data, index, a->d_err);
-            k_headers_casc<MS_FMT_FOR_DVBP><<<grid, 256, 0, st>>>(nb, L, bws, prefix, refs, data);
-            break;
-        }
-        MS_CUDA_TRY(cudaGetLastError());
-    }
-    k_finish_sizes<<<1, 32, 0, st>>>(nb, L, bws, prefix, d_compr);
-    MS_CUDA_TRY(cudaGetLastError());
-    const uint64_t nrest = n - ncompr;
-    if (nrest) {
-        k_copy_rest<<<(unsigned)minu((nrest + 255) / 256, 1024), 256, 0, st>>>(d_in + ncompr, nrest, fmt, L.bw,
-                                                                                     d_compr, data);
-        MS_CUDA_TRY(cudaGetLastError());
-    }
     uint64_t compr = 0;
-    MS_CUDA_TRY(cudaMemcpyAsync(&compr, d_compr, 8, cudaMemcpyDeviceToHost, st));
+    if (nb && fmt == MS_FMT_STATIC_VBP) {
+        compr = nb * 64ull * L.bw;
+        k_pack_static<<<grid, 256, 0, st>>>(d_in, nb, L.bw, data, a->d_err);
+        MS_CUDA_TRY(cudaGetLastError());
+    } else if (nb) {
+        const uint64_t ntiles = (nb + kEncBlocks - 1) / kEncBlocks, nwords = ntiles * kRdWordStride;
+        index = arena_take_t<uint64_t>(a, nb + 1);
+        if (fmt == MS_FMT_FOR_DVBP) refs = arena_take_t<uint64_t>(a, nb / 2 + 1);
+        unsigned *words = arena_take_t<unsigned>(a, nwords + 2);  // and the compressed size
+        if (!index || !words || (fmt == MS_FMT_FOR_DVBP && !refs)) return ms_fail(MS_ERR_NOMEM, "arena exhausted (encode scratch)");
+        d_compr = reinterpret_cast<uint64_t *>(words + nwords);
+        MS_CUDA_TRY(cudaMemsetAsync(words, 0, 4 * (nwords + 2), st));
+        auto kern = fmt == MS_FMT_DYNAMIC_VBP ? k_encode<MS_FMT_DYNAMIC_VBP>
+                    : fmt == MS_FMT_DELTA_DVBP ? k_encode<MS_FMT_DELTA_DVBP> : k_encode<MS_FMT_FOR_DVBP>;
+        int rc = launch_rounds(kern, ntiles, st, d_in, nb, L, words, data, index, refs, nrest, d_compr, a->d_err);
+        if (rc) return rc;
+        if (fmt == MS_FMT_DYNAMIC_VBP && L.dvbp_shift > 2) {
+            const unsigned page = 1u << L.dvbp_shift;
+            const uint64_t bytes = (nb + page - 1) / page * kPageBlocks;
+            k_headers_dvbp<<<unsigned(minu((bytes + 255) / 256, grid)), 256, 0, st>>>(nb, page, index, data);
+            MS_CUDA_TRY(cudaGetLastError());
+        }
+        if (fmt == MS_FMT_FOR_DVBP && L.for_shift > 1) {
+            const unsigned page = 1u << L.for_shift;
+            const uint64_t hw = (nb / 2 + page - 1) / page * 8;
+            k_headers_for<<<unsigned(minu((hw + 255) / 256, grid)), 256, 0, st>>>(nb / 2, page, index, refs, data);
+            MS_CUDA_TRY(cudaGetLastError());
+        }
+    }
+    if (nrest && (!d_compr || nrest > kEncRest)) {
+        k_copy_rest<<<(unsigned)minu((nrest + 255) / 256, 1024), 256, 0, st>>>(d_in + ncompr, nrest, fmt, L.bw, d_compr,
+                                                                               compr, data);
+        MS_CUDA_TRY(cudaGetLastError());
+    }
+    if (d_compr) MS_CUDA_TRY(cudaMemcpyAsync(&compr, d_compr, 8, cudaMemcpyDeviceToHost, st));
     int rc = read_err(a, st);  // synchronises
     if (rc) return rc;
     *out = ms_col{};
@@ -1022,7 +1134,7 @@ static int encode(const uint64_t *d_in, uint64_t n, uint64_t ncompr, Layout L, m
     out->size_alloc_byte = cap;
     out->data = data;
     out->index = index;
-    out->index_aux = aux;
+    out->index_aux = refs;
     out->n_index = index ? nb : 0;
     return MS_OK;
 }
@@ -1045,7 +1157,7 @@ int compress_values(const uint64_t *d_in, uint64_t n, int fmt, unsigned bw, ms_c
     if (fmt == MS_FMT_STATIC_VBP && (bw < 1 || bw > 64)) return ms_fail(MS_ERR_INVALID, "static_vbp bw must be 1..64");
     if (fmt < 0 || fmt > MS_FMT_RLE) return ms_fail(MS_ERR_INVALID, "unknown format");
     const uint64_t b = block_size(fmt);
-    Layout L{fmt, bw, kPageBlocks, kForPageBlocks};
+    Layout L{fmt, bw, 6, 3};  // 64 blocks, 8 cascade blocks a page
     return encode(d_in, n, n / b * b, L, out, a, st);
 }
 
@@ -1068,7 +1180,7 @@ int write_values(const uint64_t *d_vals, uint64_t n_vec, uint64_t n_scalar, int 
     const uint64_t b = block_size(fmt);
     const uint64_t full = n_vec / kWiBuffer * kWiBuffer;
     const uint64_t ncompr = full + (n_vec - full) / b * b;
-    Layout L{fmt, bw, kWiBuffer / kBlock, kWiBuffer / kCascBlock};
+    Layout L{fmt, bw, 2, 1};  // 2048 values a page
     return encode(d_vals, n, ncompr, L, out, a, st);
 }
 

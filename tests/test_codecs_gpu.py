@@ -217,3 +217,30 @@ def test_rle_decode_reports_inconsistent_lengths(ms, arena, orc, mean_log2, delt
     with pytest.raises(ms.MorphStoreError) as e:
         ms.morph(col, ms.uncompr_f)
     assert e.value.status == 5
+
+
+def _all_widths(orc, n, seed):
+    """Every bit width 1..64 block after block (neighbours differ)."""
+    bw = (np.arange(n // 512 + 1, dtype=np.uint64) * np.uint64(27)) % np.uint64(64) + np.uint64(1)
+    return orc.uniform_bits(seed, 64, n) >> np.repeat(np.uint64(64) - bw, 512)[:n]
+
+
+# one tile is 6144 rows; 148 tiles make a round
+@pytest.mark.parametrize("fmt", [O.DYNAMIC_VBP, O.DELTA_DVBP, O.FOR_DVBP])
+@pytest.mark.parametrize("n", [6143, 6144, 6145, 8192, 9 * 6144 + 1024, 148 * 6144, 148 * 6144 + 512, 149 * 6144 + 1535,
+                               5 * 148 * 6144 + 7 * 1024 + 3, 6 * 148 * 6144 - 1])
+def test_encode_rounds_bytes(ms, arena, orc, fmt, n):
+    """The one-pass encoder over the edges of tiles and rounds, every width,
+    against the oracle: as a morph and through the write iterator."""
+    v = _all_widths(orc, n, n)
+    col = ms.Column.from_numpy(v, arena)
+    c = ms.morph(col, _fmt(ms, fmt, 0))
+    b, m = orc.compress(fmt, 0, v)
+    assert c.meta() == m
+    assert np.array_equal(_masked(fmt, 0, c.raw_bytes(), m, orc), _masked(fmt, 0, b, m, orc))
+    assert np.array_equal(c.to_numpy(), v)
+    w = ms.project(col, ms.Column.from_numpy(np.arange(n, dtype=np.uint64), arena), _fmt(ms, fmt, 0))
+    b, m = orc.wi_write(fmt, 0, v, n % 8)
+    assert w.meta() == m
+    assert np.array_equal(_masked(fmt, 0, w.raw_bytes(), m, orc), _masked(fmt, 0, b, m, orc))
+    assert np.array_equal(w.to_numpy(), v)
