@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kRdThreads, 1)
     if (threadIdx.x == 0) {
         for (unsigned r = 0; r < kRdBufs; r++) load(r);
     }
-    RdPrefix pre(words, ntiles);
+    RdPrefix<false> pre(words, ntiles);
     for (unsigned r = 0; r <= rounds + 1; r++) {
         const uint64_t t = tile_of(r);
         if (first_half && t < ntiles) {
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kRdThreads, 1)
             rd_bar(0);  // every value of the tile is in registers
             if (w == kRdWarps - 1) {
                 const unsigned sum = __reduce_add_sync(0xFFFFFFFFu, lane < nblk ? s_bw[par][lane] : 0u);
-                if (lane == 0) rd_publish(words, t, sum);
+                if (lane == 0) rd_publish(words, t, sum, 0);
             }
             if (mine) pack_half_rt(bw, x, blk, l, h);
         }
@@ -331,301 +331,195 @@ __global__ void __launch_bounds__(256, 3) k_decode_all(ColView c, uint64_t *__re
 }
 
 // --- rle ----------------------------------------------------------------------
-// Encoder: one pass over the input in tiles of kRleTile rows, tiles taken in
-// order from a ticket counter.  A row starts a run (a "head") when it differs
-// from the row before (rle.h:63-150: maximal runs).  Each tile needs the
-// number of runs before it (its first head's run index) and the row of the
-// last head before it (where the run its first head ends began): both come
-// from a decoupled look-back over the tiles before it (every tile publishes
-// its own run count and last head, then -- once known -- the inclusive
-// values).  Every head writes its run's value and the length of the run
-// before it; the last tile writes the length of the final run.  So the input
-// is read once and each pair written once (8 B/row + 16 B/run).
-constexpr unsigned kRleEncThreads = 1024;
-constexpr unsigned kRleRowsPerThread = 16;
-constexpr unsigned kRleEncTile = kRleEncThreads * kRleRowsPerThread;  // rows per encoder tile
-constexpr uint64_t kRleNone = ~uint64_t(0);
-enum : unsigned { kRleFlagAgg = 1, kRleFlagInc = 2 };
+// Encoder: one pass in rounds (rounds.cuh).  A row starts a run (a "head") when
+// it differs from the row before (rle.h:63-150: maximal runs).  The analysing
+// warps find a tile's heads (one ballot per 32 rows) and publish their number
+// and the last one; the writing warps get from the words before the tile the
+// number of runs before it and the row where the run that its first head ends
+// began.  Every head writes the pair of the run it ends (the value of the row
+// before it, its length), the column's last tile also the final run.  So the
+// input is read once and each pair written once (8 B/row + 16 B/run).  2^26
+// rows, mean run 32: 149 us (208 with a look-back by CTAs that load, search,
+// look back and write one after another; 87 at the copy rate); runs of one
+// row 350 us a call (373), of 1000 rows 188 us (226).
+__global__ void __launch_bounds__(kRdThreads, 1)
+    k_rle_encode(const uint64_t *__restrict__ in, uint64_t n, unsigned *words, ulonglong2 *__restrict__ out,
+                 uint64_t *__restrict__ d_runs, unsigned *err) {
+    extern __shared__ __align__(128) uint8_t rd_smem[];
+    __shared__ RdShared sh;
+    __shared__ unsigned s_heads[kRdBufs][kRdRows / 32];  // by buffer: heads of 32 rows
+    __shared__ unsigned s_cnt[kRdWarps], s_last[kRdWarps];
+    const unsigned tid = threadIdx.x % kRdHalf, w = tid >> 5, lane = tid & 31u;
+    const bool first_half = threadIdx.x < kRdHalf;
+    const uint64_t ntiles = (n + kRdRows - 1) / kRdRows;
+    const unsigned rounds = unsigned((ntiles + gridDim.x - 1) / gridDim.x);
+    auto tile_of = [&](unsigned r) { return uint64_t(r) * gridDim.x + blockIdx.x; };
+    auto rows_of = [&](uint64_t t) { return unsigned(minu(kRdRows, n - t * kRdRows)); };
+    auto load = [&](unsigned r) {
+        const uint64_t t = tile_of(r);
+        if (t < ntiles)
+            rd_load(rd_buf(rd_smem, r), sh.full + r % kRdBufs, in, t * kRdRows, rows_of(t), t ? 2u : 0u);
+    };
+    rd_init(sh);
+    if (threadIdx.x == 0) {
+        for (unsigned r = 0; r < kRdBufs; r++) load(r);
+    }
+    RdPrefix<true> pre(words, ntiles);
+    for (unsigned r = 0; r <= rounds + 1; r++) {
+        const uint64_t t = tile_of(r);
+        if (first_half && t < ntiles) {
+            const unsigned rows = rows_of(t);
+            uint64_t *const v = reinterpret_cast<uint64_t *>(rd_buf(rd_smem, r) + kRdHead);
+            rd_full(sh, r);
+            if (rows & 1u) {  // the column's odd last row
+                if (tid == 0) v[rows - 1] = __ldg(in + n - 1);
+                rd_bar(0);
+            }
+            // warp w: rows [1024 w, 1024 (w + 1)); lane k keeps word k
+            unsigned mine = 0;
+#pragma unroll 8
+            for (unsigned k = 0; k < 32; k++) {
+                const unsigned i = 1024u * w + 32u * k + lane;
+                const bool head = i < rows && (t + i == 0 || v[i] != v[int(i) - 1]);
+                const unsigned b = __ballot_sync(0xFFFFFFFFu, head);
+                if (k == lane) mine = b;
+            }
+            s_heads[r % kRdBufs][32 * w + lane] = mine;
+            const unsigned cnt = __reduce_add_sync(0xFFFFFFFFu, __popc(mine));
+            const unsigned last = __reduce_max_sync(0xFFFFFFFFu, mine ? 1024u * w + 32u * lane + 32u - __clz(mine) : 0u);
+            if (lane == 0) {
+                s_cnt[w] = cnt;
+                s_last[w] = last;
+            }
+            rd_bar(0);
+            if (tid == 0) {
+                unsigned c = 0, z = 0;
+                for (unsigned i = 0; i < kRdWarps; i++) {
+                    c += s_cnt[i];
+                    z = max(z, s_last[i]);
+                }
+                rd_publish(words, t, c, z);
+            }
+        }
+        if (!first_half && r && r <= rounds) pre.request(r - 1, tid);  // read in the next round
+        if (!first_half && r > 1) {
+            const uint64_t tp = tile_of(r - 2);
+            pre.sums(sh, r - 2, tid);
+            if (tp < ntiles) {
+                const uint64_t *const v = reinterpret_cast<const uint64_t *>(rd_buf(rd_smem, r - 2) + kRdHead);
+                const unsigned *const heads = s_heads[(r - 2) % kRdBufs];
+                // runs before the warp's first word, the head before it
+                unsigned before = 0, prev = 0;  // prev: row of the tile + 1, 0 for none in the tile
+                for (unsigned i = lane; i < 32 * w; i += 32) {
+                    const unsigned x = heads[i];
+                    before += __popc(x);
+                    if (x) prev = 32u * i + 32u - __clz(x);
+                }
+                before = __reduce_add_sync(0xFFFFFFFFu, before);
+                prev = __reduce_max_sync(0xFFFFFFFFu, prev);
+                const unsigned word = heads[32 * w + lane], c = __popc(word);
+                unsigned incl = c, lastw = word ? 1024u * w + 32u * lane + 32u - __clz(word) : 0u;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const unsigned o = __shfl_up_sync(0xFFFFFFFFu, incl, d), z = __shfl_up_sync(0xFFFFFFFFu, lastw, d);
+                    if (int(lane) >= d) {
+                        incl += o;
+                        lastw = max(lastw, z);
+                    }
+                }
+                const unsigned tot = __shfl_sync(0xFFFFFFFFu, incl, 31), tail = max(prev, __shfl_sync(0xFFFFFFFFu, lastw, 31));
+                unsigned ph = __shfl_up_sync(0xFFFFFFFFu, lastw, 1);  // the head before the lane's word
+                ph = max(prev, lane ? ph : 0u);
+                const uint64_t row0 = tp * kRdRows, run0 = pre.base + pre.lower + before;
+                // the pair that the head at tile row i ends: run `run` of the
+                // column, which began at the head before, p (+ 1, 0: before the tile)
+                auto put = [&](uint64_t run, unsigned i, unsigned p) {
+                    if (run) out[run - 1] = make_ulonglong2(v[int(i) - 1], row0 + i + 1 - (p ? row0 + p : pre.last));
+                };
+                if (__reduce_max_sync(0xFFFFFFFFu, c) > 20) {
+                    // nearly all rows are heads: a warp per word, consecutive
+                    // lanes write consecutive pairs; else a lane per word,
+                    // which takes as many steps as its word has heads
+                    for (unsigned k = 0; k < 32; k++) {
+                        const unsigned x = __shfl_sync(0xFFFFFFFFu, word, k), o = __shfl_sync(0xFFFFFFFFu, incl - c, k);
+                        const unsigned p = __shfl_sync(0xFFFFFFFFu, ph, k), below = x & ((1u << lane) - 1u);
+                        const unsigned i = 1024u * w + 32u * k;
+                        if ((x >> lane) & 1u) put(run0 + o + __popc(below), i + lane, below ? i + 32u - __clz(below) : p);
+                    }
+                } else {
+                    uint64_t run = run0 + (incl - c);
+                    unsigned p = ph;
+                    for (unsigned x = word; x; x &= x - 1) {
+                        const unsigned i = 1024u * w + 32u * lane + unsigned(__ffs(x) - 1);
+                        put(run++, i, p);
+                        p = i + 1;
+                    }
+                }
+                if (tp == ntiles - 1 && w == kRdWarps - 1 && lane == 0) {
+                    // the final run ends at row n
+                    const uint64_t total = run0 + tot;
+                    *d_runs = total;
+                    out[total - 1] = make_ulonglong2(v[n - row0 - 1], n + 1 - (tail ? row0 + tail : pre.last));
+                }
+            }
+            pre.next();
+            fence_async_smem();  // the buffer's last accesses, before a bulk copy overwrites it
+            rd_bar(1);
+            if (tid == 0) load(r + 2);
+        }
+        if (first_half) fence_async_smem();
+        else pre.turn();
+        __syncthreads();
+    }
+    if (sh.fail && threadIdx.x == 0) atomicOr(err, kErrTimeout);
+}
 
-// A tile's published values in two 64-bit words, each carrying the flag in
-// its low two bits (0: nothing yet, kRleFlagAgg: the tile's own values,
-// kRleFlagInc: the values over tiles [0, this tile]): r = runs << 2 | flag,
-// l = (last head + 1, 0 for none) << 2 | flag.  Each word is written and
-// read whole, so a value is never seen without its flag and no fence is
-// needed; a reader that sees the two words with different flags (one
-// already updated) reads again.
-struct RleTileState {
-    unsigned long long r, l;
+// The short-run decoder's tiles find the rows before them by a decoupled
+// look-back over the tiles before (every tile publishes its own row count,
+// then -- once known -- the inclusive one).
+// A tile's published count carries the flag in its low two bits (0: nothing
+// yet, kRleFlagAgg: the tile's own rows, kRleFlagInc: the rows of tiles [0,
+// this tile]): written and read whole, so no fence is needed.  It has a cache
+// line of its own (rounds.cuh).
+enum : unsigned { kRleFlagAgg = 1, kRleFlagInc = 2 };
+struct __align__(128) RleTileState {
+    unsigned long long r;
 };
 
-__device__ __forceinline__ void rle_publish(RleTileState *s, unsigned flag, uint64_t runs, uint64_t last) {
-    const unsigned long long r = (runs << 2) | flag;
-    const unsigned long long l = ((last == kRleNone ? 0 : last + 1) << 2) | flag;
-    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(s), "l"(r), "l"(l) : "memory");
+__device__ __forceinline__ void rle_publish(RleTileState *s, unsigned flag, uint64_t rows) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&s->r), "l"((rows << 2) | flag) : "memory");
 }
 
 // Warp-wide look-back (warp 0 of the tile): lane i inspects tile j - i, 32
-// predecessors per step, with one 16-byte load per lane and step; the
-// nearest one with an inclusive prefix ends the walk.  Returns false if a
-// predecessor never published (bounded spin).
-__device__ bool rle_lookback(const RleTileState *state, uint64_t tile, uint64_t &excl_runs, uint64_t &excl_last) {
+// predecessors per step; the nearest one with an inclusive count ends the
+// walk.  Returns false if a predecessor never published (bounded spin).
+__device__ bool rle_lookback(const RleTileState *state, uint64_t tile, uint64_t &excl) {
     const unsigned lane = threadIdx.x & 31u;
-    excl_runs = 0;
-    excl_last = kRleNone;
+    excl = 0;
     for (int64_t j = int64_t(tile) - 1; j >= 0; j -= 32) {
         const int64_t me = j - int64_t(lane);
-        unsigned f = kRleFlagInc;  // lanes before tile 0 act as an empty inclusive prefix
-        uint64_t cr = 0, cl = kRleNone;
+        unsigned long long r = kRleFlagInc;  // lanes before tile 0 act as an empty inclusive prefix
         if (me >= 0) {
-            const RleTileState *o = state + me;
-            unsigned long long r = 0, l = 0;
             for (unsigned spins = 0; spins < kSpinLimit; spins++) {
-                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(r), "=l"(l) : "l"(o) : "memory");
-                if ((r & 3u) != 0 && (r & 3u) == (l & 3u)) break;
+                asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(r) : "l"(&state[me].r) : "memory");
+                if (r & 3u) break;
             }
-            f = (r & 3u) == (l & 3u) ? unsigned(r & 3u) : 0u;
-            cr = r >> 2;
-            cl = (l >> 2) ? (l >> 2) - 1 : kRleNone;
         }
+        const unsigned f = unsigned(r & 3u);
         if (__any_sync(0xFFFFFFFFu, f == 0)) return false;
         const unsigned inc = __ballot_sync(0xFFFFFFFFu, f == kRleFlagInc);
         const unsigned stop = inc ? unsigned(__ffs(inc) - 1) : 32u;  // lanes 0..stop count
-        const bool take = lane <= stop;
-        uint64_t r = take ? cr : 0;
+        uint64_t s = lane <= stop ? r >> 2 : 0;
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) r += __shfl_xor_sync(0xFFFFFFFFu, r, d);
-        excl_runs += r;
-        if (excl_last == kRleNone) {
-            // the nearest taken predecessor with a head
-            const unsigned has = __ballot_sync(0xFFFFFFFFu, take && cl != kRleNone);
-            if (has) excl_last = __shfl_sync(0xFFFFFFFFu, cl, __ffs(has) - 1);
-        }
+        for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, d);
+        excl += s;
         if (inc) break;
     }
     return true;
 }
 
-__global__ void __launch_bounds__(kRleEncThreads) k_rle_encode(const uint64_t *__restrict__ in, uint64_t n,
-                                                              RleTileState *state, unsigned *ticket,
-                                                              uint64_t *__restrict__ out,
-                                                              uint64_t *__restrict__ d_runs, unsigned *err) {
-    constexpr unsigned NW = kRleEncThreads / 32, WR = 32 * kRleRowsPerThread;  // warps, rows per warp
-    __shared__ uint64_t s_tile;
-    __shared__ unsigned s_wcnt[NW];
-    __shared__ uint64_t s_wlast[NW];
-    __shared__ uint64_t s_excl_runs, s_excl_last;
-    const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-    __syncthreads();
-    const uint64_t tile = s_tile;
-    const uint64_t ntiles = (n + kRleEncTile - 1) / kRleEncTile;
-    if (tile >= ntiles) return;
-    // warp w covers WR consecutive rows; in step k lane l reads row base + 32 k + l
-    // (one coalesced 256-byte load per step); heads as one ballot per step
-    const uint64_t base = tile * kRleEncTile + uint64_t(wid) * WR;
-    uint64_t carry = base > 0 && base <= n ? __ldg(in + base - 1) : 0;  // the row before the step's first
-    unsigned ball[kRleRowsPerThread];
-    unsigned c = 0;
-#pragma unroll
-    for (unsigned k = 0; k < kRleRowsPerThread; k++) {
-        const uint64_t r = base + 32 * k + lane;
-        const uint64_t v = r < n ? __ldg(in + r) : 0;
-        const uint64_t up = __shfl_up_sync(0xFFFFFFFFu, v, 1);
-        const uint64_t prev = lane ? up : carry;
-        carry = __shfl_sync(0xFFFFFFFFu, v, 31);
-        ball[k] = __ballot_sync(0xFFFFFFFFu, r < n && (r == 0 || v != prev));
-        c += __popc(ball[k]);
-    }
-    // last head of this warp as row + 1 (0: none)
-    uint64_t my_last = 0;
-#pragma unroll
-    for (unsigned k = 0; k < kRleRowsPerThread; k++)
-        if (ball[k]) my_last = base + 32 * k + (31 - __clz(ball[k])) + 1;
-    if (lane == 0) {
-        s_wcnt[wid] = c;
-        s_wlast[wid] = my_last;
-    }
-    __syncthreads();
-    unsigned wpre = 0;
-    uint64_t wlast = 0;
-    for (unsigned w = 0; w < wid; w++) {
-        wpre += s_wcnt[w];
-        wlast = maxu(wlast, s_wlast[w]);
-    }
-    if (wid == 0) {
-        // the whole tile: runs and last head; publish, then look back
-        uint64_t agg_runs = 0, agg_last = 0;
-        for (unsigned w = 0; w < NW; w++) {
-            agg_runs += s_wcnt[w];
-            agg_last = maxu(agg_last, s_wlast[w]);
-        }
-        RleTileState *me = state + tile;
-        const uint64_t own_last = agg_last ? agg_last - 1 : kRleNone;
-        uint64_t excl_runs = 0, excl_last = kRleNone;
-        if (tile == 0) {
-            if (lane == 0) rle_publish(me, kRleFlagInc, agg_runs, own_last);
-        } else {
-            if (lane == 0) rle_publish(me, kRleFlagAgg, agg_runs, own_last);
-            __syncwarp();
-            if (!rle_lookback(state, tile, excl_runs, excl_last) && lane == 0) atomicOr(err, kErrTimeout);
-            if (lane == 0)
-                rle_publish(me, kRleFlagInc, excl_runs + agg_runs, own_last != kRleNone ? own_last : excl_last);
-        }
-        if (lane == 0) {
-            s_excl_runs = excl_runs;
-            s_excl_last = excl_last;
-            if (tile == ntiles - 1) {
-                // the final run ends at row n
-                const uint64_t total = excl_runs + agg_runs;
-                const uint64_t last = own_last != kRleNone ? own_last : excl_last;
-                *d_runs = total;
-                if (total) out[2 * (total - 1) + 1] = n - last;
-            }
-        }
-    }
-    __syncthreads();
-    // pairs: every head writes its run's value and the length of the run
-    // before it; consecutive lanes write consecutive pairs
-    uint64_t k_run = s_excl_runs + wpre;                       // run index of the warp's next head
-    uint64_t prev_head = wlast ? wlast - 1 : s_excl_last;      // row of the head before it
-    const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-    for (unsigned k = 0; k < kRleRowsPerThread; k++) {
-        const unsigned bk = ball[k];
-        if (!bk) continue;
-        const uint64_t r = base + 32 * k + lane;
-        if ((bk >> lane) & 1u) {
-            const uint64_t idx = k_run + __popc(bk & below);
-            const unsigned lower = bk & below;
-            const uint64_t ph = lower ? base + 32 * k + (31 - __clz(lower)) : prev_head;
-            out[2 * idx] = __ldg(in + r);
-            if (idx) out[2 * (idx - 1) + 1] = r - ph;
-        }
-        k_run += __popc(bk);
-        prev_head = base + 32 * k + (31 - __clz(bk));
-    }
-}
-
-// Staged encoder: the same algorithm, one tile of kRleStThreads *
-// kRleRowsPerThread rows per CTA, with the tile's rows brought into shared
-// memory by asynchronous 16-byte copies (cp.async) that are all in flight at
-// once instead of one register load per step; each lane compares its row
-// with the one before it in shared memory.  Three CTAs per SM, so one CTA's
-// look-back overlaps the others' reads.  Needs a 16-byte aligned input.
-constexpr unsigned kRleStThreads = 512;
-constexpr unsigned kRleStTile = kRleStThreads * kRleRowsPerThread;
-
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
-__global__ void __launch_bounds__(kRleStThreads) k_rle_encode_staged(const uint64_t *__restrict__ in, uint64_t n,
-                                                                    RleTileState *state, unsigned *ticket,
-                                                                    uint64_t *__restrict__ out,
-                                                                    uint64_t *__restrict__ d_runs, unsigned *err) {
-    constexpr unsigned NW = kRleStThreads / 32, WR = 32 * kRleRowsPerThread;
-    extern __shared__ __align__(128) uint8_t rle_smem[];
-    uint64_t *const v = reinterpret_cast<uint64_t *>(rle_smem);  // the tile's rows
-    __shared__ uint64_t s_tile;
-    __shared__ unsigned s_ball[NW][kRleRowsPerThread];
-    __shared__ unsigned s_wcnt[NW];
-    __shared__ uint64_t s_wlast[NW];
-    __shared__ uint64_t s_excl_runs, s_excl_last;
-    const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-    __syncthreads();
-    const uint64_t tile = s_tile;
-    const uint64_t ntiles = (n + kRleStTile - 1) / kRleStTile;
-    if (tile >= ntiles) return;
-    const uint64_t r0 = tile * kRleStTile;
-    const unsigned rows = unsigned(minu(kRleStTile, n - r0));
-    {
-        // every 16-byte pair of rows of the tile, consecutive threads on
-        // consecutive pairs; an odd last row of the column is read directly
-        const unsigned pairs = rows / 2;
-        for (unsigned q = threadIdx.x; q < pairs; q += kRleStThreads) cp_async16(v + 2 * q, in + r0 + 2 * q);
-        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-        if ((rows & 1u) && threadIdx.x == 0) v[rows - 1] = __ldg(in + r0 + rows - 1);
-    }
-    __syncthreads();
-    // heads: warp w covers tile rows [w WR, (w + 1) WR), lane-strided; the
-    // tile's first row is compared with the previous tile's last
-    const unsigned wbase = wid * WR;
-    const uint64_t before = r0 ? __ldg(in + r0 - 1) : 0;
-    unsigned c = 0;
-    uint64_t my_last = 0;  // last head of this warp as row + 1 (0: none)
-#pragma unroll
-    for (unsigned k = 0; k < kRleRowsPerThread; k++) {
-        const unsigned lr = wbase + 32 * k + lane;
-        const bool valid = lr < rows;
-        const uint64_t x = valid ? v[lr] : 0;
-        const uint64_t prev = lr ? v[lr - 1] : before;
-        const unsigned bk = __ballot_sync(0xFFFFFFFFu, valid && (r0 + lr == 0 || x != prev));
-        if (lane == 0) s_ball[wid][k] = bk;
-        c += __popc(bk);
-        if (bk) my_last = r0 + wbase + 32 * k + (31 - __clz(bk)) + 1;
-    }
-    if (lane == 0) {
-        s_wcnt[wid] = c;
-        s_wlast[wid] = my_last;
-    }
-    __syncthreads();
-    if (wid == 0) {
-        // the whole tile: runs and last head; publish, then look back
-        uint64_t agg_runs = lane < NW ? s_wcnt[lane] : 0, agg_last = lane < NW ? s_wlast[lane] : 0;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            agg_runs += __shfl_xor_sync(0xFFFFFFFFu, agg_runs, d);
-            agg_last = maxu(agg_last, __shfl_xor_sync(0xFFFFFFFFu, agg_last, d));
-        }
-        RleTileState *me = state + tile;
-        const uint64_t own_last = agg_last ? agg_last - 1 : kRleNone;
-        uint64_t excl_runs = 0, excl_last = kRleNone;
-        if (tile > 0) {
-            if (lane == 0) rle_publish(me, kRleFlagAgg, agg_runs, own_last);
-            __syncwarp();
-            if (!rle_lookback(state, tile, excl_runs, excl_last) && lane == 0) atomicOr(err, kErrTimeout);
-        }
-        if (lane == 0) {
-            rle_publish(me, kRleFlagInc, excl_runs + agg_runs, own_last != kRleNone ? own_last : excl_last);
-            s_excl_runs = excl_runs;
-            s_excl_last = excl_last;
-            if (tile == ntiles - 1) {
-                // the final run ends at row n
-                const uint64_t total = excl_runs + agg_runs;
-                const uint64_t last = own_last != kRleNone ? own_last : excl_last;
-                *d_runs = total;
-                if (total) out[2 * (total - 1) + 1] = n - last;
-            }
-        }
-    }
-    __syncthreads();
-    // pairs: every head writes its run's value and the length of the run
-    // before it; consecutive lanes write consecutive pairs
-    unsigned wpre = 0;
-    uint64_t wlast = 0;
-    for (unsigned w = 0; w < wid; w++) {
-        wpre += s_wcnt[w];
-        wlast = maxu(wlast, s_wlast[w]);
-    }
-    uint64_t k_run = s_excl_runs + wpre;                   // run index of the warp's next head
-    uint64_t prev_head = wlast ? wlast - 1 : s_excl_last;  // row of the head before it
-    const unsigned below = (1u << lane) - 1u;
-#pragma unroll 4
-    for (unsigned k = 0; k < kRleRowsPerThread; k++) {
-        const unsigned bk = s_ball[wid][k];
-        if (!bk) continue;
-        const unsigned lr = wbase + 32 * k + lane;
-        if ((bk >> lane) & 1u) {
-            const uint64_t idx = k_run + __popc(bk & below);
-            const unsigned lower = bk & below;
-            const uint64_t ph = lower ? r0 + wbase + 32 * k + (31 - __clz(lower)) : prev_head;
-            out[2 * idx] = v[lr];
-            if (idx) out[2 * (idx - 1) + 1] = r0 + lr - ph;
-        }
-        k_run += __popc(bk);
-        prev_head = r0 + wbase + 32 * k + (31 - __clz(bk));
-    }
 }
 
 constexpr unsigned kRleThreads = 256;
@@ -907,12 +801,12 @@ __global__ void __launch_bounds__(kRleLbThreads, 2) k_rle_expand_lb(const uint64
     }
     // publish the tile's rows, then the rows before it
     RleTileState *me = state + tile;
-    if (threadIdx.x == 0 && tile > 0) rle_publish(me, kRleFlagAgg, agg, kRleNone);
+    if (threadIdx.x == 0 && tile > 0) rle_publish(me, kRleFlagAgg, agg);
     if (wid == 0) {
-        uint64_t excl = 0, unused = kRleNone;
-        if (tile > 0 && !rle_lookback(state, tile, excl, unused) && lane == 0) atomicOr(err, kErrTimeout);
+        uint64_t excl = 0;
+        if (tile > 0 && !rle_lookback(state, tile, excl) && lane == 0) atomicOr(err, kErrTimeout);
         if (lane == 0) {
-            rle_publish(me, kRleFlagInc, excl + agg, kRleNone);
+            rle_publish(me, kRleFlagInc, excl + agg);
             s_base = excl;
             if (tile == ntiles - 1 && excl + agg != n) atomicOr(err, kErrCorrupt);
         }
@@ -973,32 +867,38 @@ __global__ void __launch_bounds__(kRleLbThreads, 2) k_rle_expand_lb(const uint64
 // ---------------------------------------------------------------------------
 // host drivers
 // ---------------------------------------------------------------------------
+// Launch of a rounds kernel: one CTA per SM at most, all resident.
+template <class... P, class... A>
+static int launch_rounds(void (*kern)(P...), uint64_t ntiles, cudaStream_t st, A... args) {
+    constexpr size_t smem = kRdSmem;
+    MS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    lc.gridDim = dim3(unsigned(minu(ntiles, uint64_t(sm_count()))));
+    lc.blockDim = dim3(kRdThreads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    MS_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, P(args)...));
+    return MS_OK;
+}
+
 static int encode_rle(const uint64_t *d_in, uint64_t n, ms_col *out, ms_arena *a, cudaStream_t st) {
-    // tile states for the smaller of the two encoders' tiles
-    const uint64_t tiles = (n + minu(kRleEncTile, kRleStTile) - 1) / minu(kRleEncTile, kRleStTile);
+    const uint64_t tiles = (n + kRdRows - 1) / kRdRows, nwords = tiles * kRdWordStride;
     uint8_t *data = arena_take_t<uint8_t>(a, 16 * n + 64);
-    RleTileState *state = arena_take_t<RleTileState>(a, tiles + 1);
-    unsigned *ticket = arena_take_t<unsigned>(a, 2);
-    uint64_t *d_runs = arena_take_t<uint64_t>(a, 1);
-    if (!data || !state || !ticket || !d_runs) return ms_fail(MS_ERR_NOMEM, "arena exhausted (rle)");
+    unsigned *words = arena_take_t<unsigned>(a, nwords + 2);  // and the number of runs
+    if (!data || !words) return ms_fail(MS_ERR_NOMEM, "arena exhausted (rle)");
     uint64_t runs = 0;
     if (n) {
-        MS_CUDA_TRY(cudaMemsetAsync(state, 0, sizeof(RleTileState) * tiles, st));
-        MS_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));
-        if ((reinterpret_cast<uintptr_t>(d_in) & 15u) == 0) {
-            // rows staged in shared memory (16-byte aligned input)
-            constexpr size_t smem = size_t(kRleStTile) * 8;
-            MS_CUDA_TRY(cudaFuncSetAttribute(k_rle_encode_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(smem)));
-            k_rle_encode_staged<<<unsigned((n + kRleStTile - 1) / kRleStTile), kRleStThreads, smem, st>>>(
-                d_in, n, state, ticket, (uint64_t *)data, d_runs, a->d_err);
-        } else {
-            k_rle_encode<<<unsigned((n + kRleEncTile - 1) / kRleEncTile), kRleEncThreads, 0, st>>>(
-                d_in, n, state, ticket, (uint64_t *)data, d_runs, a->d_err);
-        }
-        MS_CUDA_TRY(cudaGetLastError());
+        uint64_t *d_runs = reinterpret_cast<uint64_t *>(words + nwords);
+        MS_CUDA_TRY(cudaMemsetAsync(words, 0, 4 * (nwords + 2), st));
+        int rc = launch_rounds(k_rle_encode, tiles, st, d_in, n, words, (ulonglong2 *)data, d_runs, a->d_err);
+        if (rc) return rc;
         MS_CUDA_TRY(cudaMemcpyAsync(&runs, d_runs, 8, cudaMemcpyDeviceToHost, st));
-        int rc = read_err(a, st);  // synchronises the stream
+        rc = read_err(a, st);  // synchronises the stream
         if (rc) return rc;
     }
     *out = ms_col{};
@@ -1054,25 +954,6 @@ static int decode_rle(const ms_col *in, uint64_t *d_out, ms_arena *a, cudaStream
     default: k_rle_expand<8><<<unsigned(chunks), kRleThreads, 0, st>>>(pairs, runs, tfirst, tiles, ctile, tot, n, d_out, a->d_err); break;
     }
     MS_CUDA_TRY(cudaGetLastError());
-    return MS_OK;
-}
-
-// Launch of a rounds kernel: one CTA per SM at most, all resident.
-template <class... P, class... A>
-static int launch_rounds(void (*kern)(P...), uint64_t ntiles, cudaStream_t st, A... args) {
-    constexpr size_t smem = kRdSmem;
-    MS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    cudaLaunchConfig_t lc = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    lc.gridDim = dim3(unsigned(minu(ntiles, uint64_t(sm_count()))));
-    lc.blockDim = dim3(kRdThreads);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = st;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    MS_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, P(args)...));
     return MS_OK;
 }
 

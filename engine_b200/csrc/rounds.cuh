@@ -47,7 +47,7 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 
 struct RdShared {
     uint64_t full[kRdBufs];
-    unsigned lower[kRdWarps], total[kRdWarps];
+    unsigned lower[kRdWarps], total[kRdWarps], lower_last[kRdWarps], total_last[kRdWarps];
     volatile unsigned fail;
 };
 
@@ -73,14 +73,17 @@ __device__ __forceinline__ void rd_load(uint8_t *buf, uint64_t *full, const uint
                                         unsigned before) {
     const unsigned bytes = 8u * ((rows & ~1u) + before);
     mbar_arrive_expect_tx(full, bytes);
-    bulk_g2s(buf + kRdHead - 8u * before, in + row0 - before, bytes, full);
+    if (bytes) bulk_g2s(buf + kRdHead - 8u * before, in + row0 - before, bytes, full);
 }
 
 // Published words, one per tile, each in a line of its own (neighbours in one
 // line made a word some 5 us late: the line is written by many SMs while
-// others read it): bit 0 set, the payload above it.
+// others read it): bit 0 set, above it 13 bits that are summed up (block
+// widths, runs) and 13 bits of which the latest counts (last run head + 1, 0
+// for none).
 constexpr unsigned kRdWordStride = 32;
-__device__ __forceinline__ void rd_publish(unsigned *words, uint64_t tile, unsigned payload) {
+__device__ __forceinline__ void rd_publish(unsigned *words, uint64_t tile, unsigned sum, unsigned last) {
+    const unsigned payload = last << 13 | sum;
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(words + tile * kRdWordStride), "r"(payload << 1 | 1u)
                  : "memory");
 }
@@ -90,14 +93,18 @@ __device__ __forceinline__ unsigned rd_peek(const unsigned *w) {
     return x;
 }
 
-// Sums over the words of a round: `base` = the rounds before it, `lower` = the
-// round's tiles before the CTA's, by the output half.
+// What a tile needs from the words before it, by the output half: `base` =
+// the sum over the rounds before, `lower` = over the round's tiles before the
+// CTA's; kLast: `last` = the latest position before the tile (row + 1).
+template <bool kLast>
 struct RdPrefix {
     const unsigned *words;
     uint64_t ntiles;
-    uint64_t base = 0;
-    unsigned lower = 0, total = 0;
+    uint64_t base = 0, last = 0;
+    unsigned lower = 0;
     unsigned cur = 0, nxt = 0;
+    unsigned total = 0;       // of the round
+    uint64_t base_last = 0;   // latest position in the rounds before
 
     __device__ RdPrefix(const unsigned *w, uint64_t n) : words(w), ntiles(n) {}
 
@@ -113,28 +120,49 @@ struct RdPrefix {
     }
     __device__ __forceinline__ void sums(RdShared &sh, unsigned r, unsigned tid) {
         const unsigned n = in_round(r);
-        unsigned lo = 0, to = 0;
+        unsigned lo = 0, to = 0, llo = 0, lto = 0;
         for (unsigned i = tid; i < n; i += kRdHalf) {
             unsigned x = i == tid ? cur : 0u;
             for (unsigned spins = 0; !(x & 1u) && !sh.fail; spins++) {
                 if (spins >= kSpinLimit) sh.fail = 1;
                 x = rd_peek(word(r, i));
             }
-            to += x >> 1;
-            lo += i < blockIdx.x ? x >> 1 : 0u;
+            const unsigned sum = (x >> 1) & 0x1FFFu, at = x >> 14 ? i << 13 | x >> 14 : 0u;
+            to += sum;
+            lo += i < blockIdx.x ? sum : 0u;
+            lto = max(lto, at);
+            llo = max(llo, i < blockIdx.x ? at : 0u);
         }
         lo = __reduce_add_sync(0xFFFFFFFFu, lo);
         to = __reduce_add_sync(0xFFFFFFFFu, to);
+        if (kLast) {
+            llo = __reduce_max_sync(0xFFFFFFFFu, llo);
+            lto = __reduce_max_sync(0xFFFFFFFFu, lto);
+        }
         if ((tid & 31u) == 0) {
             sh.lower[tid >> 5] = lo;
             sh.total[tid >> 5] = to;
+            if (kLast) {
+                sh.lower_last[tid >> 5] = llo;
+                sh.total_last[tid >> 5] = lto;
+            }
         }
         rd_bar(1);
         lower = total = 0;
+        llo = lto = 0;
 #pragma unroll
         for (unsigned i = 0; i < kRdWarps; i++) {
             lower += sh.lower[i];
             total += sh.total[i];
+            if (kLast) {
+                llo = max(llo, sh.lower_last[i]);
+                lto = max(lto, sh.total_last[i]);
+            }
+        }
+        if (kLast) {
+            const auto row1 = [&](unsigned at) { return (uint64_t(r) * gridDim.x + (at >> 13)) * kRdRows + (at & 0x1FFFu); };
+            last = llo ? row1(llo) : base_last;
+            if (lto) base_last = row1(lto);
         }
     }
     __device__ __forceinline__ void next() { base += total; }

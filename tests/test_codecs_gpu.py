@@ -244,3 +244,19 @@ def test_encode_rounds_bytes(ms, arena, orc, fmt, n):
     assert w.meta() == m
     assert np.array_equal(_masked(fmt, 0, w.raw_bytes(), m, orc), _masked(fmt, 0, b, m, orc))
     assert np.array_equal(w.to_numpy(), v)
+
+
+@pytest.mark.parametrize("mean_log2", [0, 2, 5, 14])
+@pytest.mark.parametrize("n", [1, 2, 3, 6143, 6144, 6145, 2 * 6144 + 1, 148 * 6144 - 1, 148 * 6144 + 1, 3 * 148 * 6144 + 31])
+def test_rle_encode_rounds(ms, arena, orc, mean_log2, n):
+    """Runs within and across tiles and rounds, tiles without a head, an odd
+    last row, words with few and with many heads."""
+    v = orc.runs(n + mean_log2, mean_log2, 20, n) if mean_log2 else orc.uniform_bits(n, 20, n)
+    c = ms.morph(ms.Column.from_numpy(v, arena), ms.rle_f)
+    b, m = orc.compress(O.RLE, 0, v)
+    assert c.meta() == m
+    assert np.array_equal(c.raw_bytes(), b[: m[1]])
+    assert np.array_equal(c.to_numpy(), v)
+    one = np.full(n, 9, np.uint64)  # a single run
+    c = ms.morph(ms.Column.from_numpy(one, arena), ms.rle_f)
+    assert c.meta() == (n, 16, 16) and c.raw_bytes().view(np.uint64).tolist() == [9, n]
