@@ -260,3 +260,18 @@ def test_rle_encode_rounds(ms, arena, orc, mean_log2, n):
     one = np.full(n, 9, np.uint64)  # a single run
     c = ms.morph(ms.Column.from_numpy(one, arena), ms.rle_f)
     assert c.meta() == (n, 16, 16) and c.raw_bytes().view(np.uint64).tolist() == [9, n]
+
+
+@pytest.mark.parametrize("bits", [0, 4, 26, 27, 28, 33, 64])
+@pytest.mark.parametrize("n", [1024, 1024 + 7, 3552 * 512, 3552 * 512 + 1024, 2 * 3552 * 512 + 1024 + 513])
+def test_delta_segments(ms, arena, orc, bits, n):
+    """Segments of one and of several blocks per warp, deltas on both sides of
+    the 32-bit sums' limit; the carries of every block (through select) and
+    the lane sums of the column."""
+    v = orc.sorted_gaps(n, orc.geom_table(0.25), n) if bits == 0 else np.cumsum(orc.uniform_bits(n + bits, bits, n), dtype=np.uint64)
+    b, m = orc.compress(O.DELTA_DVBP, 0, v)
+    c = ms.Column.from_bytes(ms.delta_f, b, m, arena)
+    assert np.array_equal(c.to_numpy(), v)
+    assert ms.agg_sum(c) == orc.agg_sum(v)
+    lanes = v[: n // 1024 * 1024].reshape(-1, 8)[-1]
+    assert np.array_equal(c.delta_lane_sums(), lanes)
