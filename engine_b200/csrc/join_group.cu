@@ -285,59 +285,89 @@ __global__ void __launch_bounds__(kSmem ? 32 * kProbeWarps : 256, kSmem ? 1 : 3)
     if (!ok) atomicOr(err, kErrCorrupt);
 }
 
-// intersect: rows of l (a sorted position list) whose value occurs in the
-// sorted array rv; pass structure as k_probe, output = the values.
-__global__ void __launch_bounds__(256) k_intersect(ColView lc, const uint64_t *__restrict__ rv, uint64_t nr,
-                                                  uint32_t *__restrict__ blk_counts, const uint64_t *__restrict__ blk_off,
-                                                  uint64_t *__restrict__ out, unsigned long long *__restrict__ d_scalar,
-                                                  unsigned *err) {
-    const unsigned lane = threadIdx.x & 31u, l = lane & 7u, q = lane >> 3;
-    bool ok = true;
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < lc.nblocks_total();
-         b += uint64_t(gridDim.x) * blockDim.x / 32) {
-        uint64_t v[16];
-        unsigned valid;
-        ok &= decode_block(lc, b, l, q, v, valid);
-        unsigned m = 0;
-        // the thread's 16 values ascend: galloping lower-bound searches
-        uint64_t j = 0;
+// intersect, pass 1: hit bits = rows of l (a sorted position list) whose value
+// occurs in the sorted array rv; the hits' values compact per block.  A warp
+// finds the part of rv that its block's values span by two 32-way searches,
+// copies it to shared memory when it has at most kIsectPart values, and runs
+// the binary searches of a thread's 16 values side by side in it (in rv
+// itself when the part is longer).
+constexpr unsigned kIsectPart = 1024;
+
+// first index in rv[lo, hi) with rv[i] >= x (kUpper: > x); all lanes together
+template <bool kUpper>
+__device__ __forceinline__ uint64_t warp_bound(const uint64_t *__restrict__ rv, uint64_t lo, uint64_t hi, uint64_t x,
+                                               unsigned lane) {
+    while (lo < hi) {
+        const uint64_t step = (hi - lo + 31) / 32, p = lo + lane * step;
+        const bool before = p < hi && (kUpper ? __ldg(rv + p) <= x : __ldg(rv + p) < x);
+        const unsigned cnt = __popc(__ballot_sync(0xFFFFFFFFu, before));  // probes before the bound: a prefix
+        if (cnt == 0) return lo;
+        const uint64_t last = lo + (cnt - 1) * step;
+        hi = minu(hi, last + step);
+        lo = last + 1;
+    }
+    return lo;
+}
+
+// bit k: v[k] occurs in the sorted a[0, len), len > 0
+template <class I>
+__device__ __forceinline__ unsigned search16(const uint64_t *a, I len, const uint64_t (&v)[16]) {
+    I at[16];
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            if (!((valid >> k) & 1u)) continue;
-            const uint64_t x = v[k];
-            uint64_t step = 1, lo = j, hi = j;
-            while (hi < nr && rv[hi] < x) {
-                lo = hi + 1;
-                hi = j + step;
-                step <<= 1;
-            }
-            if (hi > nr) hi = nr;
-            while (lo < hi) {
-                const uint64_t mid = (lo + hi) >> 1;
-                if (rv[mid] < x) lo = mid + 1;
-                else hi = mid;
-            }
-            j = lo;
-            if (j < nr && rv[j] == x) m |= 1u << k;
-        }
-        if (!blk_off) {
-            const unsigned tot = __reduce_add_sync(0xFFFFFFFFu, __popc(m));
-            if (lane == 0) blk_counts[b] = tot;
-            continue;
-        }
-        if (!__any_sync(0xFFFFFFFFu, m != 0)) continue;
-        unsigned rank[16];
-        block_ranks(m, l, q, rank);
-        const uint64_t base = blk_off[b], row0 = b * kBlock;
-        unsigned scal = 0;
+    for (int k = 0; k < 16; k++) at[k] = 0;
+    for (I n = len; n > 1;) {
+        const I h = n >> 1;
+#pragma unroll
+        for (int k = 0; k < 16; k++) at[k] += a[at[k] + h - 1] < v[k] ? h : 0;
+        n -= h;
+    }
+    unsigned m = 0;
+#pragma unroll
+    for (int k = 0; k < 16; k++) m |= unsigned(a[at[k]] == v[k]) << k;
+    return m;
+}
+
+__global__ void __launch_bounds__(256, 3) k_intersect_bits(ColView lc, const uint64_t *__restrict__ rv, uint64_t nr,
+                                                          MaskRun run, uint64_t *__restrict__ side, unsigned *err) {
+    extern __shared__ __align__(16) uint64_t isect_smem[];
+    uint64_t *const part = isect_smem + (threadIdx.x >> 5) * kIsectPart;
+    bool ok = true;
+    mask_pass(run, [&](uint64_t b, unsigned l, unsigned q) -> unsigned {
+        const unsigned lane = threadIdx.x & 31u;
+        uint64_t v[16];
+        unsigned valid, m = 0;
+        ok &= decode_block(lc, b, l, q, v, valid);
+        // the block's last value: the largest of the valid ones
+        uint64_t hi_v = 0;
 #pragma unroll
         for (int k = 0; k < 16; k++)
-            if ((m >> k) & 1u) {
-                out[base + rank[k]] = v[k];
-                scal += (row0 + (16u * q + k) * 8u + l) >= lc.sfrom;
+            if ((valid >> k) & 1u) hi_v = maxu(hi_v, v[k]);
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) hi_v = maxu(hi_v, __shfl_xor_sync(0xFFFFFFFFu, hi_v, d));
+        const uint64_t lo_v = __shfl_sync(0xFFFFFFFFu, v[0], 0);
+        const uint64_t lo = warp_bound<false>(rv, 0, nr, lo_v, lane), hi = warp_bound<true>(rv, lo, nr, hi_v, lane);
+        if (lo < hi) {
+            const uint64_t len = hi - lo;
+            if (len <= kIsectPart) {
+                for (unsigned i = lane; i < len; i += 32) part[i] = __ldg(rv + lo + i);
+                __syncwarp();
+                m = search16<unsigned>(part, unsigned(len), v);
+            } else {
+                m = search16<uint64_t>(rv + lo, len, v);
             }
-        if (scal) atomicAdd(d_scalar, (unsigned long long)scal);
-    }
+            m &= valid;
+            __syncwarp();  // the part is free for the warp's next block
+        }
+        if (__any_sync(0xFFFFFFFFu, m != 0)) {
+            uint64_t *const o = side + (b - run.b0) * kBlock;
+            unsigned rank[16];
+            block_ranks(m, l, q, rank);
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                if ((m >> k) & 1u) o[rank[k]] = v[k];
+        }
+        return m;
+    });
     if (!ok) atomicOr(err, kErrCorrupt);
 }
 
@@ -706,38 +736,6 @@ static unsigned grid_blocks(uint64_t nbt) {
     return (unsigned)maxu(1, minu((nbt + 7) / 8, persistent_grid(256, 8)));
 }
 
-// Shared tail of position-producing operators: pass 1 counts, scan, pass 2
-// writes; then the write iterator model.
-template <class Launch>
-static int positions_two_pass(uint64_t nbt, Launch launch, int out_format, unsigned out_bw, ms_col *out, ms_arena *a,
-                              cudaStream_t st) {
-    uint32_t *bc = arena_take_t<uint32_t>(a, nbt + 1);
-    uint64_t *bo = arena_take_t<uint64_t>(a, nbt + 1);
-    uint64_t *tot = arena_take_t<uint64_t>(a, 2);
-    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(nbt, 1));
-    if (!bc || !bo || !tot || !scr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions)");
-    MS_CUDA_TRY(cudaMemsetAsync(tot, 0, 16, st));
-    if (nbt) {
-        launch(bc, nullptr, nullptr, nullptr);
-        MS_CUDA_TRY(cudaGetLastError());
-        MS_CUDA_TRY((scan_exclusive<uint32_t, 1>(bc, nbt, bo, tot, scr, st)));
-    }
-    uint64_t total = 0;
-    MS_CUDA_TRY(cudaMemcpyAsync(&total, tot, 8, cudaMemcpyDeviceToHost, st));
-    MS_CUDA_TRY(cudaStreamSynchronize(st));
-    uint64_t *pos = arena_take_t<uint64_t>(a, total + 1);
-    if (!pos) return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions output)");
-    if (total) {
-        launch(bc, bo, pos, (unsigned long long *)(tot + 1));
-        MS_CUDA_TRY(cudaGetLastError());
-    }
-    uint64_t scal = 0;
-    MS_CUDA_TRY(cudaMemcpyAsync(&scal, tot + 1, 8, cudaMemcpyDeviceToHost, st));
-    int rc = read_err(a, st);
-    if (rc) return rc;
-    return write_values(pos, total - scal, scal, out_format, out_bw, out, a, st);
-}
-
 // The bitmap goes to shared memory when it fits and the probe side is long
 // enough to pay for each SM's copy: an SM copies `words` and then looks up
 // its share of the rows, one word each.
@@ -833,7 +831,7 @@ extern "C" int ms_gpu_semi_join(const ms_col *l, const ms_col *r, int out_format
             k_probe_bits<false><<<mask_grid(run.nblk, 8, 3), 256, 0, st>>>(rv, s, run, a->d_err);
     };
     uint64_t *pos, cnt, nscal;
-    rc = rows_by_mask<false, uint32_t>(rv, pass1, &pos, nullptr, &cnt, &nscal, a, st);
+    rc = rows_by_mask<kRows, uint32_t>(rv, pass1, &pos, nullptr, &cnt, &nscal, a, st);
     if (rc) return rc;
     return write_values(pos, cnt - nscal, nscal, out_format, out_bw, out, a, st);
 }
@@ -857,11 +855,16 @@ extern "C" int ms_gpu_intersect_sorted(const ms_col *l, const ms_col *r, int out
         rc = check_col(r, false);
         if (rc) return rc;
     }
-    const uint64_t nr = r->count_values, nbt = lv.nblocks_total();
-    auto launch = [&](uint32_t *bc, const uint64_t *bo, uint64_t *pos, unsigned long long *scal) {
-        k_intersect<<<grid_blocks(nbt), 256, 0, st>>>(lv, rvals, nr, bc, bo, pos, scal, a->d_err);
+    const uint64_t nr = r->count_values;
+    constexpr size_t smem = 8 * size_t(kIsectPart) * 8;
+    MS_CUDA_TRY(cudaFuncSetAttribute(k_intersect_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    auto pass1 = [&](const MaskRun &run, uint64_t *side) {
+        k_intersect_bits<<<mask_grid(run.nblk, 8, 3), 256, smem, st>>>(lv, rvals, nr, run, side, a->d_err);
     };
-    return positions_two_pass(nbt, launch, out_format, out_bw, out, a, st);
+    uint64_t *vals, cnt, nscal;
+    rc = rows_by_mask<kVals, uint64_t>(lv, pass1, nullptr, &vals, &cnt, &nscal, a, st);
+    if (rc) return rc;
+    return write_values(vals, cnt - nscal, nscal, out_format, out_bw, out, a, st);
 }
 
 extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format, ms_col *out_gr, int ext_format,
@@ -1091,7 +1094,7 @@ extern "C" int ms_gpu_natural_join(const ms_col *l, const ms_col *r, int out_l_f
             else
                 k_probe_map_bits<false, V><<<mask_grid(run.nblk, 8, 3), 256, 0, st>>>(rv, m, run, side, a->d_err);
         };
-        return rows_by_mask<true, V>(rv, pass1, &pr, &pl, &total, &scal, a, st);
+        return rows_by_mask<kRows | kVals, V>(rv, pass1, &pr, &pl, &total, &scal, a, st);
     };
     rc = nl < 0xFFFFFFFFull ? join(uint32_t(0)) : join(uint64_t(0));
     if (rc) return rc;

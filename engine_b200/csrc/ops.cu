@@ -339,7 +339,7 @@ extern "C" int ms_gpu_select(int cmp, uint64_t val, const ms_col *in, int out_fo
     auto pass1 = [&](const MaskRun &r, uint32_t *) {
         k_select_bits<<<mask_grid(r.nblk, 8, 4), 256, 0, st>>>(x, cmp, val, pred, r, a->d_err);
     };
-    rc = rows_by_mask<false, uint32_t>(x, pass1, &pos, nullptr, &cnt, &nscal, a, st);
+    rc = rows_by_mask<kRows, uint32_t>(x, pass1, &pos, nullptr, &cnt, &nscal, a, st);
     if (rc) return rc;
     return write_values(pos, cnt - nscal, nscal, out_format, out_bw, out, a, st);
 }

@@ -92,13 +92,17 @@ inline unsigned mask_grid(uint64_t nblk, unsigned warps, unsigned ctas_per_sm) {
     return (unsigned)maxu(1, minu((nblk + warps - 1) / warps, maxu(persistent_grid(32 * warps, ctas_per_sm), 128)));
 }
 
-// Pass 2: positions (and with kVals the compact per-block values of pass 1:
-// block i's j-th hit at side[i * 512 + j]) from *base_in on; the last unit
+// What an operator gives per hit: the row's position, a value of its own
+// (compact per block in `side`), or both.
+enum : int { kRows = 1, kVals = 2 };
+
+// Pass 2: positions and / or the compact per-block values of pass 1 (block
+// i's j-th hit at side[i * 512 + j]) from *base_in on; the last unit
 // stores the end in *base_out.  Words with many hits are written by a warp
 // each (consecutive lanes, consecutive addresses), sparse ones by a lane
 // each.  Nothing is written at or beyond index `cap`.  scalar: hits at rows
 // >= sfrom.
-template <bool kVals, class V>
+template <int kOut, class V>
 __global__ void __launch_bounds__(256) k_expand_rows(MaskRun r, uint64_t n, uint64_t sfrom,
                                                     const unsigned long long *__restrict__ base_in,
                                                     unsigned long long *__restrict__ base_out, uint64_t cap,
@@ -143,7 +147,8 @@ __global__ void __launch_bounds__(256) k_expand_rows(MaskRun r, uint64_t n, uint
         const uint64_t wbase = base + pre;             // the warp's first output
         const uint64_t row = r.b0 * kBlock + wi * 32;  // the word's first row
         if (wtot && wbase + wtot <= cap) {
-            if (wtot > 128) {
+            if (!(kOut & kRows)) {
+            } else if (wtot > 128) {
 #pragma unroll 4
                 for (int i = 0; i < 32; i++) {
                     const uint32_t x = __shfl_sync(0xFFFFFFFFu, word, i);
@@ -155,7 +160,7 @@ __global__ void __launch_bounds__(256) k_expand_rows(MaskRun r, uint64_t n, uint
                 uint64_t *o = out + wbase + (incl - c);
                 for (uint32_t x = word; x; x &= x - 1) *o++ = row + unsigned(__ffs(x) - 1);
             }
-            if (kVals) {
+            if (kOut & kVals) {
                 // the warp's two blocks
                 const unsigned c0 = __shfl_sync(0xFFFFFFFFu, incl, 15), c1 = wtot - c0;
                 const V *s = side + (w0 + 32ull * warp) / kBlockWords * kBlock;
@@ -191,29 +196,29 @@ struct TopScratch {
     }
 };
 
-// The driver.  pass1(run, side): launches pass 1 over run's blocks.  kVals:
-// the operator also gives one value per hit (side: V per hit, compact per
-// block); the output size is then read back before pass 2, so that both
-// outputs are exactly as long as they have to be, while positions alone are
-// written into the free rest of the arena and trimmed.  A column whose bits
+// The driver.  pass1(run, side): launches pass 1 over run's blocks.  With two
+// outputs their size is read back before pass 2, so that both are exactly as
+// long as they have to be, while a single one is written into the free rest
+// of the arena and trimmed.  A column whose bits
 // do not fit is done in segments of blocks; short of memory, a segment takes
 // no more than 11 bytes per block of the column.
-template <bool kVals, class V, class Pass1>
+template <int kOut, class V, class Pass1>
 int rows_by_mask(const ColView &x, Pass1 pass1, uint64_t **d_pos, uint64_t **d_vals, uint64_t *count,
                  uint64_t *n_scalar, ms_arena *a, cudaStream_t st) {
     const uint64_t nbt = x.nblocks_total(), n = x.n;
-    const uint64_t per = 64 + (kVals ? kBlock * sizeof(V) : 0);  // bytes per block
+    constexpr bool kBoth = kOut == (kRows | kVals);
+    const uint64_t per = 64 + (kOut & kVals ? kBlock * sizeof(V) : 0);  // bytes per block
     TopScratch ts(a);
     unsigned long long *words = ts.take<unsigned long long>(4);  // running base (two words), remainder hits
     if (!words) return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions)");
     uint64_t seg = nbt;
-    if (per * nbt + (kVals ? 16 : 8) * n + 4 * kMaxUnits + 4096 > ts.room())
+    if (per * nbt + (kBoth ? 16 : 8) * n + 4 * kMaxUnits + 4096 > ts.room())
         seg = maxu(1, minu(nbt, 11 * nbt / per));
     const unsigned unit = mask_unit(seg);
     unsigned *counts = ts.take<unsigned>((seg + unit - 1) / maxu(unit, 1) + 1);
     uint32_t *bits = ts.take<uint32_t>(seg * kBlockWords);
-    V *side = kVals ? ts.take<V>(seg * kBlock) : nullptr;
-    if (!counts || !bits || (kVals && !side)) return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions)");
+    V *side = kOut & kVals ? ts.take<V>(seg * kBlock) : nullptr;
+    if (!counts || !bits || ((kOut & kVals) && !side)) return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions)");
     MS_CUDA_TRY(cudaMemsetAsync(words, 0, 32, st));
     auto run_of = [&](uint64_t b0) {
         MaskRun r{b0, minu(seg, nbt - b0), unit, 0, bits, counts};
@@ -229,7 +234,7 @@ int rows_by_mask(const ColView &x, Pass1 pass1, uint64_t **d_pos, uint64_t **d_v
     uint64_t cap = 0, total = 0;
     uint64_t *pos = nullptr, *vals = nullptr;
     std::vector<unsigned> h;
-    if (kVals) {
+    if (kBoth) {
         for (uint64_t b0 = 0; b0 < nbt; b0 += seg) {
             const MaskRun r = run_of(b0);
             int rc = first(r);
@@ -245,16 +250,16 @@ int rows_by_mask(const ColView &x, Pass1 pass1, uint64_t **d_pos, uint64_t **d_v
         cap = total;
     } else {
         cap = minu(n, ts.room() / 8);
-        pos = reinterpret_cast<uint64_t *>(a->base + align_up(a->used, 256));
+        pos = vals = reinterpret_cast<uint64_t *>(a->base + align_up(a->used, 256));
     }
     unsigned ping = 0;
     for (uint64_t b0 = 0; b0 < nbt; b0 += seg, ping ^= 1u) {
         const MaskRun r = run_of(b0);
-        if (!kVals || seg < nbt) {  // else the bits are there already
+        if (!kBoth || seg < nbt) {  // else the bits are there already
             int rc = first(r);
             if (rc) return rc;
         }
-        k_expand_rows<kVals, V><<<r.nunits, 256, 0, st>>>(r, n, x.sfrom, words + ping, words + (ping ^ 1u), cap, pos,
+        k_expand_rows<kOut, V><<<r.nunits, 256, 0, st>>>(r, n, x.sfrom, words + ping, words + (ping ^ 1u), cap, pos,
                                                           side, vals, words + 2);
         MS_CUDA_TRY(cudaGetLastError());
     }
@@ -262,13 +267,13 @@ int rows_by_mask(const ColView &x, Pass1 pass1, uint64_t **d_pos, uint64_t **d_v
     MS_CUDA_TRY(cudaMemcpyAsync(hw, words, 24, cudaMemcpyDeviceToHost, st));
     int rc = read_err(a, st);
     if (rc) return rc;
-    if (!kVals) {
+    if (!kBoth) {
         total = hw[ping];
         if (total > cap || !arena_take_t<uint64_t>(a, total + 1))
             return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions output)");
     }
-    *d_pos = pos;
-    if (kVals) *d_vals = vals;
+    if (kOut & kRows) *d_pos = pos;
+    if (kOut & kVals) *d_vals = vals;
     *count = total;
     *n_scalar = hw[2];
     return MS_OK;

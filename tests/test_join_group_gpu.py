@@ -199,3 +199,18 @@ def test_group_counts_around_table_limits(ms, arena, orc, groups, fmt):
     egr2, eext2 = orc.group(k2, egr)
     assert np.array_equal(ext2.to_numpy(), eext2)
     assert np.array_equal(gr2.to_numpy(), egr2)
+
+
+@pytest.mark.parametrize("nl,nr,l_gap,r_gap", [(1, 1, 1, 1), (513, 4097, 1, 1), (5000, 70_000, 16, 1), (70_000, 5000, 1, 16),
+                                               (3000, 400_000, 200, 1), (400_003, 300_001, 1, 1), (20_000, 7, 1, 4096)])
+@pytest.mark.parametrize("code", [O.UNCOMPR, O.DELTA_DVBP])
+def test_intersect_parts(ms, arena, orc, nl, nr, l_gap, r_gap, code):
+    """A block of the left side that spans few, many (over 1024) and no values
+    of the right one; disjoint ranges; hits at both ends."""
+    def col(seed, n, gap):
+        return np.cumsum(orc.uniform_bits(seed, 20, n) % np.uint64(2 * gap) + np.uint64(1), dtype=np.uint64)
+    a, b = col(nl, nl, l_gap), col(nr + 1, nr, r_gap)
+    b[-1] = max(int(b[-1]), int(a[-1]))
+    for r in (b, b + np.uint64(int(a[-1]) + 1)):
+        out = ms.intersect_sorted(_col(ms, arena, orc, a, code), _col(ms, arena, orc, r, code))
+        assert np.array_equal(out.to_numpy(), orc.intersect_sorted(a, r))
