@@ -290,7 +290,9 @@ __global__ void __launch_bounds__(kSmem ? 32 * kProbeWarps : 256, kSmem ? 1 : 3)
 // finds the part of rv that its block's values span by two 32-way searches,
 // copies it to shared memory when it has at most kIsectPart values, and runs
 // the binary searches of a thread's 16 values side by side in it (in rv
-// itself when the part is longer).
+// itself when the part is longer).  Two lists of 2^22.7 positions: 74 us, and
+// 7 to collect the values; galloping searches in global memory, one value
+// after another in two passes, took 401.
 constexpr unsigned kIsectPart = 1024;
 
 // first index in rv[lo, hi) with rv[i] >= x (kUpper: > x); all lanes together

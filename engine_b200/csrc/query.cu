@@ -25,6 +25,7 @@
 #include "scan.cuh"
 #include "stream.cuh"
 #include "tma.cuh"
+#include "window.cuh"
 
 namespace ms {
 namespace {
@@ -148,14 +149,21 @@ __global__ void __launch_bounds__(256) k_query3(ColView filt, ColView fk, ColVie
 // Staged variant.  One persistent CTA per SM: warp 0 forms tiles of
 // consecutive 512-row blocks whose bytes in all four fact columns fit one
 // stage buffer and brings each column's range into shared memory with one
-// bulk copy; consumer warps take the tile's blocks round-robin.  Per block
-// the filter is decoded and compared inside the bit-width switch (all 512
-// rows); the foreign key, group key and measure are not decoded as blocks:
-// only the values of rows still alive are extracted from the staged words
-// (about 10%, 1% and 1% of the rows in the star query), so the consumers stay
-// below the memory time.  Requires the filter in uncompr/static_vbp/
-// dynamic_vbp and the other three columns in those or for_f (delta_f and
-// rows in the uncompressed rests go through k_query3).
+// bulk copy; consumer warps take the tile's blocks two at a time, round-robin.
+// The filter is compared inside the bit-width switch (32 rows per thread) and
+// the hits of both blocks are listed, so that their foreign keys are extracted
+// and probed 128 at a time, four per lane, every lane busy; the rows that
+// survive are compacted in the list, their group key and measure extracted
+// together and queued per warp, and 32 queued rows at a time go to the CTA's
+// group table.  The producer takes block locations from windows it loaded
+// ahead (window.cuh) and forms a tile before it waits for its stage: its path
+// per tile bounded the pass.  2^27 rows: 293 us (356 before; 412 with the
+// listed hits alone), of which reading the columns takes 149; the rest is the
+// consumers' instructions at 17 warps per SM (24 warps leave a smaller ring:
+// 383 us).
+// Requires the filter in uncompr/static_vbp/dynamic_vbp and the other three
+// columns in those or for_f (delta_f and rows in the uncompressed rests go
+// through k_query3).
 // ---------------------------------------------------------------------------
 constexpr unsigned kQTile = 32;  // blocks per tile (one producer lane each)
 constexpr unsigned kQCols = 4;   // filter, fk, group key, measure
@@ -171,9 +179,55 @@ struct QCfg {
     unsigned stage_bytes;
 };
 
-// value of slot s (0..63) of lane l in a vbp block of width bw
-__device__ __forceinline__ uint64_t vbp_extract(const uint64_t *blk, unsigned bw, unsigned l, unsigned s) {
-    const unsigned p = s * bw, w = p >> 6, sh = p & 63u;
+// A consumer warp's list of hits (rows of its two blocks) and queue of rows to be
+// grouped (kQQueue entries: up to 31 left over and 32 new ones).
+constexpr unsigned kQQueue = 64;
+struct QWarp {
+    unsigned long long key[kQQueue], val[kQQueue], row[kQQueue];
+    uint16_t hits[2 * kBlock];  // second block << 9 | row
+};
+
+// The CTA's group table: sums as two 32-bit words (32-bit shared atomics are
+// native).
+struct QTable {
+    unsigned long long *key, *first;
+    unsigned *lo, *hi;
+};
+
+// Folds one row into the CTA's table, or into the global one when the key
+// finds no place among 16 slots.  A key that is there with a smaller row
+// costs two loads and one atomic.
+__device__ __forceinline__ bool qtable_add(const QTable &t, const GTable &gt, uint64_t key, uint64_t row, uint64_t val) {
+    if (key != kQEmpty) {
+        unsigned h = unsigned(qhash(key)) & (kQSlots - 1);
+        for (unsigned p = 0; p < 16; p++) {
+            unsigned long long x = ((volatile unsigned long long *)t.key)[h];
+            if (x == kQEmpty) x = atomicCAS(t.key + h, kQEmpty, (unsigned long long)key);
+            if (x == kQEmpty || x == key) {
+                if (row < ((volatile unsigned long long *)t.first)[h]) atomicMin(t.first + h, (unsigned long long)row);
+                const unsigned lo = unsigned(val), old = lo ? atomicAdd(t.lo + h, lo) : 0u;
+                const unsigned hi = unsigned(val >> 32) + (old + lo < old ? 1u : 0u);
+                if (hi) atomicAdd(t.hi + h, hi);
+                return true;
+            }
+            h = (h + 1) & (kQSlots - 1);
+        }
+    }
+    return gtable_add(gt, key, row, val);
+}
+
+// value of row r (0..511) of a vbp block of width bw staged in shared memory;
+// for widths up to 32 from the two 32-bit words at its first bit (the second
+// one may lie up to 64 bytes behind the block, within shared memory)
+__device__ __forceinline__ uint64_t vbp_extract(const uint64_t *blk, unsigned bw, unsigned r) {
+    const unsigned l = r & 7u, p = (r >> 3) * bw;
+    if (bw <= 32u) {
+        const uint32_t *const b = reinterpret_cast<const uint32_t *>(blk) + 2u * l;
+        const unsigned i = p >> 5, j = i + 1u;
+        const uint32_t x = __funnelshift_r(b[(i >> 1) * 16u + (i & 1u)], b[(j >> 1) * 16u + (j & 1u)], p & 31u);
+        return bw == 32u ? x : x & ((1u << bw) - 1u);
+    }
+    const unsigned w = p >> 6, sh = p & 63u;
     uint64_t x = blk[w * 8u + l] >> sh;
     if (sh + bw > 64u) x |= blk[(w + 1u) * 8u + l] << (64u - sh);
     return bw >= 64u ? x : x & ((uint64_t(1) << bw) - 1u);
@@ -228,17 +282,19 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
     uint32_t *offs = reinterpret_cast<uint32_t *>(desc + S);                 // [S][kQCols][kQTile]
     uint8_t *bws = reinterpret_cast<uint8_t *>(offs + S * kQCols * kQTile);  // [S][kQCols][kQTile]
     uint8_t *ring = smem + q3_meta_bytes(S);
-    unsigned long long *s_key = reinterpret_cast<unsigned long long *>(ring + size_t(S) * SB);
-    unsigned long long *s_first = s_key + kQSlots;
-    unsigned long long *s_sum = s_first + kQSlots;
-
-    uint32_t *s_bits = reinterpret_cast<uint32_t *>(s_sum + kQSlots);
+    QTable tab;
+    tab.key = reinterpret_cast<unsigned long long *>(ring + size_t(S) * SB);
+    tab.first = tab.key + kQSlots;
+    tab.lo = reinterpret_cast<unsigned *>(tab.first + kQSlots);
+    tab.hi = tab.lo + kQSlots;
+    QWarp *const s_warp = reinterpret_cast<QWarp *>(tab.hi + kQSlots);
+    uint32_t *s_bits = reinterpret_cast<uint32_t *>(s_warp + W);
     const uint32_t *pbits = kSB ? s_bits : bits;
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     for (unsigned i = threadIdx.x; i < kQSlots; i += blockDim.x) {
-        s_key[i] = kQEmpty;
-        s_first[i] = ~0ull;
-        s_sum[i] = 0;
+        tab.key[i] = kQEmpty;
+        tab.first[i] = ~0ull;
+        tab.lo[i] = tab.hi[i] = 0;
     }
     const uint32_t half = uint32_t((nwords + 1) / 2);  // words per CTA in a cluster
     if (kBM == kBmShared)
@@ -263,62 +319,57 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
 
     if (warp == 0) {
         // ---------------- producer ----------------
-        const StreamCol *cols[kQCols] = {&c0, &c1, &c2, &c3};
+        const StreamCol *const cols[kQCols] = {&c0, &c1, &c2, &c3};
+        BlockWindow<kQCols> win;
+        win.init(cols, b_lo, b_hi, lane);
         uint64_t b = b_lo;
         unsigned t = 0;
         for (;; t++) {
             const unsigned st = t % S, use = t / S;
-            // the next tile's block locations are requested before waiting
-            // for its stage, so the index loads overlap the wait
-            const uint64_t blk = b + lane;
-            const bool valid = blk < b_hi;
-            uint64_t off[kQCols], len[kQCols], x0[kQCols];
+            // the tile is formed before its stage is waited for
+            const bool valid = b + lane < b_hi;
+            uint64_t off[kQCols], x0[kQCols];
+            uint32_t len[kQCols], cbase[kQCols], clen[kQCols], need = 0, acc = 0, total = 0;
             unsigned bw[kQCols];
+            win.advance(cols, b, lane);
 #pragma unroll
             for (unsigned c = 0; c < kQCols; c++) {
-                off[c] = 0;
-                bw[c] = 0;
-                if (valid) blk_loc(*cols[c], blk, off[c], bw[c]);
+                win.get(c, b, lane, off[c], bw[c]);
+                x0[c] = __shfl_sync(0xFFFFFFFFu, off[c], 0);
+                len[c] = valid ? uint32_t(off[c] - x0[c]) + 64u * bw[c] : 0u;
+                need += (len[c] + 127u) / 128u * 128u;
             }
+            const unsigned T = __popc(__ballot_sync(0xFFFFFFFFu, valid && need <= SB));
+#pragma unroll
+            for (unsigned c = 0; c < kQCols; c++) {
+                clen[c] = __shfl_sync(0xFFFFFFFFu, len[c], T ? T - 1 : 0);
+                cbase[c] = acc;
+                acc += (clen[c] + 127u) / 128u * 128u;
+                total += clen[c];
+            }
+            // lane c brings column c
+            uint64_t my_src = 0;
+            uint32_t my_len = 0, my_dst = 0;
+#pragma unroll
+            for (unsigned c = 0; c < kQCols; c++)
+                if (lane == c) {
+                    my_src = reinterpret_cast<uint64_t>(cols[c]->base) + x0[c];
+                    my_len = clen[c];
+                    my_dst = cbase[c];
+                }
             if (use > 0 && !mbar_wait(empty + st, (use - 1) & 1u)) {
                 ok = false;
                 break;
             }
-            if (b >= b_hi) {
+            if (b >= b_hi || T == 0) {  // the end, or one block larger than a stage: configuration error
                 if (lane == 0) {
+                    if (b < b_hi) atomicOr(err, kErrCapacity);
                     desc[st].nblk = 0;
                     mbar_arrive(full + st);
                 }
+                ok &= b >= b_hi;
                 t++;
                 break;
-            }
-            uint64_t need = 0;
-#pragma unroll
-            for (unsigned c = 0; c < kQCols; c++) {
-                x0[c] = __shfl_sync(0xFFFFFFFFu, off[c], 0);
-                len[c] = valid ? off[c] + 64ull * bw[c] - x0[c] : 0;
-                need += align_up(len[c], 128);
-            }
-            const bool fits = valid && need <= SB;
-            const unsigned T = __popc(__ballot_sync(0xFFFFFFFFu, fits));
-            if (T == 0) {  // one block larger than a stage: configuration error
-                if (lane == 0) {
-                    atomicOr(err, kErrCapacity);
-                    desc[st].nblk = 0;
-                    mbar_arrive(full + st);
-                }
-                ok = false;
-                t++;
-                break;
-            }
-            uint32_t cbase[kQCols];
-            uint64_t clen[kQCols];
-            uint32_t acc = 0;
-#pragma unroll
-            for (unsigned c = 0; c < kQCols; c++) {
-                clen[c] = __shfl_sync(0xFFFFFFFFu, len[c], T - 1);
-                cbase[c] = acc;
-                acc += uint32_t(align_up(clen[c], 128));
             }
             if (lane < T) {
 #pragma unroll
@@ -327,20 +378,16 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
                     bws[(st * kQCols + c) * kQTile + lane] = uint8_t(bw[c]);
                 }
             }
-            __syncwarp();
             if (lane == 0) {
-                __threadfence_block();
                 desc[st].b0 = b;
                 desc[st].nblk = T;
-                __threadfence_block();
-                uint64_t total = 0;
-#pragma unroll
-                for (unsigned c = 0; c < kQCols; c++) total += clen[c];
-                mbar_arrive_expect_tx(full + st, unsigned(total));
-#pragma unroll
-                for (unsigned c = 0; c < kQCols; c++)
-                    bulk_g2s(ring + st * SB + cbase[c], cols[c]->base + x0[c], unsigned(clen[c]), full + st);
             }
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_expect_tx(full + st, total);
+            __syncwarp();
+            if (lane < kQCols)
+                bulk_g2s(ring + st * SB + my_dst, reinterpret_cast<const uint8_t *>(my_src), my_len, full + st);
             __syncwarp();
             b += T;
         }
@@ -351,9 +398,13 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
         }
     } else {
         // ---------------- consumers ----------------
-        const unsigned cw = warp - 1, l = lane & 7u, q = lane >> 3;
-        const bool fk_for = fk.fmt == MS_FMT_FOR_DVBP, g_for = gkey.fmt == MS_FMT_FOR_DVBP,
-                   m_for = meas.fmt == MS_FMT_FOR_DVBP;
+        const unsigned cw = warp - 1, l = lane & 7u, h = (lane >> 3) & 1u, hb = lane >> 4;
+        const uint64_t *const kaux = fk.fmt == MS_FMT_FOR_DVBP ? fk.aux : nullptr;
+        const uint64_t *const gaux = gkey.fmt == MS_FMT_FOR_DVBP ? gkey.aux : nullptr;
+        const uint64_t *const maux = meas.fmt == MS_FMT_FOR_DVBP ? meas.aux : nullptr;
+        QWarp &mine = s_warp[cw];
+        unsigned queued = 0;  // rows in the warp's queue
+        unsigned turn = 0;    // pairs of the tiles before, mod W
         for (unsigned t = 0;; t++) {
             const unsigned st = t % S, use = t / S;
             if (!mbar_wait(full + st, use & 1u)) {
@@ -363,107 +414,111 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
             const unsigned T = desc[st].nblk;
             if (T == 0) break;
             const uint64_t b0 = desc[st].b0;
-            const unsigned j0 = unsigned((cw + W - (b0 - b_lo) % W) % W);
+            const unsigned pairs = (T + 1) / 2;
             const uint32_t *o = offs + st * kQCols * kQTile;
             const uint8_t *w = bws + st * kQCols * kQTile;
-            for (unsigned j = j0; j < T; j += W) {
-                const uint64_t blk = b0 + j;
-                unsigned m = mask_block_rt(w[j], reinterpret_cast<const uint64_t *>(ring + o[j]), l, q, pred, bad);
-                // semi-join probe of the surviving rows
-                if (__any_sync(0xFFFFFFFFu, m != 0)) {
-                    const uint64_t *kb = reinterpret_cast<const uint64_t *>(ring + o[kQTile + j]);
-                    const unsigned kbw = w[kQTile + j];
-                    if (kbw - 1u >= 64u) {
+            for (unsigned pr = (cw + W - turn) % W; pr < pairs; pr += W) {
+                const unsigned j = 2 * pr + hb;
+                unsigned m = 0;
+                if (j < T) {
+                    m = mask32_block_rt(w[j], reinterpret_cast<const uint64_t *>(ring + o[j]), l, h, pred, bad);
+                    if (w[kQTile + j] - 1u >= 64u || w[2 * kQTile + j] - 1u >= 64u || w[3 * kQTile + j] - 1u >= 64u) {
                         bad = true;
                         m = 0;
                     }
-                    const uint64_t kref = fk_for ? __ldg(fk.aux + (blk >> 1)) : 0;
-                    // four probes in flight per thread: the bitmap words are
-                    // requested together, then tested
-                    for (unsigned r = m; r;) {
-                        unsigned kk[4];
-                        uint32_t word[4], bit[4];
-                        bool had[4], inr[4];
+                }
+                // the hits of both blocks as a list, the first block's first
+                const unsigned n = __popc(m);
+                unsigned incl = n;
 #pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            had[i] = r != 0;
-                            kk[i] = had[i] ? unsigned(__ffs(r) - 1) : 0u;
-                            r &= r - 1;
-                            const uint64_t v = vbp_extract(kb, kbw, l, 16u * q + kk[i]) + kref;
-                            const uint64_t d = v - lo;
-                            inr[i] = had[i] && v >= lo && d < span;
-                            if (kBM == kBmCluster) {
-                                const uint32_t wi = uint32_t(d >> 5);
-                                const unsigned own = wi >= half;
-                                word[i] = inr[i] ? dsmem_ld32(s_bits, wi - own * half, own) : 0u;
-                            } else {
-                                word[i] = inr[i] ? (kSB ? pbits[d >> 5] : __ldg(pbits + (d >> 5))) : 0u;
-                            }
-                            bit[i] = unsigned(d & 31u);
-                        }
+                for (int d = 1; d < 32; d <<= 1) {
+                    const unsigned x = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                    if (int(lane) >= d) incl += x;
+                }
+                {
+                    uint16_t *at = mine.hits + (incl - n);
+                    const unsigned base = hb << 9 | h << 8 | l;
+                    for (unsigned r = m; r; r &= r - 1) *at++ = uint16_t(base + 8u * unsigned(__ffs(r) - 1));
+                }
+                const unsigned n0 = __shfl_sync(0xFFFFFFFFu, incl, 15), hits = __shfl_sync(0xFFFFFFFFu, incl, 31);
+                __syncwarp();
+                unsigned alive = 0, alive0 = 0;  // surviving rows, of the first block
+                for (unsigned h0 = 0; h0 < hits; h0 += 128) {
+                    unsigned e[4];
+                    uint32_t word[4], bit[4];
 #pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            if (had[i] && !(inr[i] && ((word[i] >> bit[i]) & 1u))) m &= ~(1u << kk[i]);
-                    }
-                }
-                const unsigned total = __reduce_add_sync(0xFFFFFFFFu, __popc(m));
-                if (lane == 0) blk_hits[blk] = total;
-                if (total == 0) continue;
-                const uint64_t *gb = reinterpret_cast<const uint64_t *>(ring + o[2 * kQTile + j]);
-                const uint64_t *mb = reinterpret_cast<const uint64_t *>(ring + o[3 * kQTile + j]);
-                const unsigned gbw = w[2 * kQTile + j], mbw = w[3 * kQTile + j];
-                if (gbw - 1u >= 64u || mbw - 1u >= 64u) {
-                    bad = true;
-                    continue;
-                }
-                const uint64_t gref = g_for ? __ldg(gkey.aux + (blk >> 1)) : 0;
-                const uint64_t mref = m_for ? __ldg(meas.aux + (blk >> 1)) : 0;
-                const uint64_t row0 = blk * kBlock;
-                for (unsigned r = m; __any_sync(0xFFFFFFFFu, r != 0); r &= r - 1) {
-                    const bool hit = r != 0;
-                    const unsigned hm = __ballot_sync(0xFFFFFFFFu, hit);
-                    if (!hit) continue;
-                    const unsigned k = __ffs(r) - 1;
-                    const uint64_t key = vbp_extract(gb, gbw, l, 16u * q + k) + gref;
-                    const uint64_t val = vbp_extract(mb, mbw, l, 16u * q + k) + mref;
-                    const uint64_t first = row0 + (16u * q + k) * 8u + l;
-                    const unsigned peers = __match_any_sync(hm, key);
-                    uint64_t sm = val, f = first;
-                    for (unsigned rest = peers; rest;) {
-                        const int src = __ffs(rest) - 1;
-                        rest &= rest - 1;
-                        const uint64_t so = __shfl_sync(peers, val, src);
-                        const uint64_t fo = __shfl_sync(peers, first, src);
-                        if (src != int(lane)) {
-                            sm += so;
-                            f = minu(f, fo);
+                    for (unsigned i = 0; i < 4; i++) {
+                        const bool in = h0 + 32u * i + lane < hits;
+                        e[i] = in ? mine.hits[h0 + 32u * i + lane] : 0u;
+                        const unsigned jj = 2 * pr + (e[i] >> 9);
+                        uint64_t v = vbp_extract(reinterpret_cast<const uint64_t *>(ring + o[kQTile + jj]), w[kQTile + jj],
+                                                 e[i] & 511u);
+                        if (kaux) v += __ldg(kaux + ((b0 + jj) >> 1));
+                        const uint64_t d = v - lo;
+                        const bool inr = in && v >= lo && d < span;
+                        if (kBM == kBmCluster) {
+                            const uint32_t wi = uint32_t(d >> 5);
+                            const unsigned own = wi >= half;
+                            word[i] = inr ? dsmem_ld32(s_bits, wi - own * half, own) : 0u;
+                        } else {
+                            word[i] = inr ? (kSB ? pbits[d >> 5] : __ldg(pbits + (d >> 5))) : 0u;
                         }
+                        bit[i] = unsigned(d & 31u);
                     }
-                    if (int(lane) != __ffs(peers) - 1) continue;
-                    uint64_t h = qhash(key) & (kQSlots - 1);
-                    bool done = false;
-                    if (key != kQEmpty) {
-                        for (unsigned p = 0; p < 16; p++) {
-                            const unsigned long long old = atomicCAS(s_key + h, kQEmpty, key);
-                            if (old == kQEmpty || old == key) {
-                                atomicMin(s_first + h, (unsigned long long)f);
-                                atomicAdd(s_sum + h, (unsigned long long)sm);
-                                done = true;
-                                break;
-                            }
-                            h = (h + 1) & (kQSlots - 1);
-                        }
+                    __syncwarp();  // the list is in registers up to here
+#pragma unroll
+                    for (unsigned i = 0; i < 4; i++) {
+                        const bool hit = (word[i] >> bit[i]) & 1u;
+                        const unsigned hm = __ballot_sync(0xFFFFFFFFu, hit), from = h0 + 32u * i;
+                        if (hit) mine.hits[alive + __popc(hm & ((1u << lane) - 1u))] = uint16_t(e[i]);
+                        alive += __popc(hm);
+                        alive0 += n0 >= from + 32u ? __popc(hm) : n0 > from ? __popc(hm & ((1u << (n0 - from)) - 1u)) : 0u;
                     }
-                    if (!done) fit &= gtable_add(gt, key, f, sm);
+                    __syncwarp();
                 }
+                if (lane < 2 && 2 * pr + lane < T) blk_hits[b0 + 2 * pr + lane] = lane ? alive - alive0 : alive0;
+                // their group keys and measures
+                for (unsigned a0 = 0; a0 < alive; a0 += 32) {
+                    const unsigned cnt = min(32u, alive - a0);
+                    if (lane < cnt) {
+                        const unsigned ee = mine.hits[a0 + lane], jj = 2 * pr + (ee >> 9), row = ee & 511u;
+                        const uint64_t blk = b0 + jj;
+                        uint64_t g = vbp_extract(reinterpret_cast<const uint64_t *>(ring + o[2 * kQTile + jj]),
+                                                 w[2 * kQTile + jj], row);
+                        uint64_t v = vbp_extract(reinterpret_cast<const uint64_t *>(ring + o[3 * kQTile + jj]),
+                                                 w[3 * kQTile + jj], row);
+                        if (gaux) g += __ldg(gaux + (blk >> 1));
+                        if (maux) v += __ldg(maux + (blk >> 1));
+                        mine.key[queued + lane] = g;
+                        mine.val[queued + lane] = v;
+                        mine.row[queued + lane] = blk * kBlock + row;
+                    }
+                    queued += cnt;
+                    __syncwarp();
+                    if (queued >= 32) {
+                        fit &= qtable_add(tab, gt, mine.key[lane], mine.row[lane], mine.val[lane]);
+                        queued -= 32;
+                        __syncwarp();
+                        if (lane < queued) {
+                            mine.key[lane] = mine.key[32 + lane];
+                            mine.val[lane] = mine.val[32 + lane];
+                            mine.row[lane] = mine.row[32 + lane];
+                        }
+                        __syncwarp();
+                    }
+                }
+                __syncwarp();  // the list is free for the next pair
             }
+            turn = (turn + pairs) % W;
             __syncwarp();
             if (lane == 0) mbar_arrive(empty + st);
         }
+        if (lane < queued) fit &= qtable_add(tab, gt, mine.key[lane], mine.row[lane], mine.val[lane]);
     }
     __syncthreads();
     for (unsigned i = threadIdx.x; i < kQSlots; i += blockDim.x)
-        if (s_key[i] != kQEmpty) fit &= gtable_add(gt, s_key[i], s_first[i], s_sum[i]);
+        if (tab.key[i] != kQEmpty)
+            fit &= gtable_add(gt, tab.key[i], tab.first[i], ((unsigned long long)tab.hi[i] << 32) + tab.lo[i]);
     if (!ok) atomicOr(err, kErrTimeout);
     if (bad) atomicOr(err, kErrCorrupt);
     if (!fit) atomicOr(err, kErrCapacity);
@@ -501,35 +556,39 @@ __global__ void __launch_bounds__(256) k_q3_extents(GTable gt, ColView filt, Col
                                                    uint64_t *__restrict__ o, unsigned *err) {
     const unsigned lane = threadIdx.x & 31u, l = lane & 7u, q = lane >> 3;
     bool ok = true;
-    for (uint64_t h = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; h <= gt.mask;
-         h += uint64_t(gridDim.x) * blockDim.x / 32) {
-        const uint64_t key = gt.keys[h];
-        if (key == kQEmpty) continue;
-        const uint64_t row = gt.first[h];
-        const uint64_t b = row / kBlock;
-        uint64_t v[16];
-        unsigned valid;
-        ok &= decode_block(filt, b, l, q, v, valid);
-        unsigned m = select_mask(filt, b, l, q, v, valid, cmp, c);
-        ok &= decode_block(fk, b, l, q, v, valid);
+    // 32 slots per warp and step, the occupied ones one after another
+    for (uint64_t h0 = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * 32; h0 <= gt.mask;
+         h0 += uint64_t(gridDim.x) * blockDim.x) {
+        const uint64_t my_key = gt.keys[h0 + lane];  // the table has a multiple of 32 slots
+        for (unsigned todo = __ballot_sync(0xFFFFFFFFu, my_key != kQEmpty); todo; todo &= todo - 1) {
+            const uint64_t h = h0 + unsigned(__ffs(todo) - 1);
+            const uint64_t key = __shfl_sync(0xFFFFFFFFu, my_key, __ffs(todo) - 1);
+            const uint64_t row = gt.first[h];
+            const uint64_t b = row / kBlock;
+            uint64_t v[16];
+            unsigned valid;
+            ok &= decode_block(filt, b, l, q, v, valid);
+            unsigned m = select_mask(filt, b, l, q, v, valid, cmp, c);
+            ok &= decode_block(fk, b, l, q, v, valid);
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const uint64_t d = v[k] - lo;
-            if (!(v[k] >= lo && d < span && ((bits[d >> 5] >> (d & 31u)) & 1u))) m &= ~(1u << k);
-        }
-        unsigned rank[16];
-        block_ranks(m, l, q, rank);
-        const unsigned s = unsigned(row % kBlock) / 8u;  // slot of the row within its lane
-        unsigned rk = 0;
+            for (int k = 0; k < 16; k++) {
+                const uint64_t d = v[k] - lo;
+                if (!(v[k] >= lo && d < span && ((bits[d >> 5] >> (d & 31u)) & 1u))) m &= ~(1u << k);
+            }
+            unsigned rank[16];
+            block_ranks(m, l, q, rank);
+            const unsigned s = unsigned(row % kBlock) / 8u;  // slot of the row within its lane
+            unsigned rk = 0;
 #pragma unroll
-        for (unsigned k = 0; k < 16; k++) rk = (16u * q + k == s) ? rank[k] : rk;
-        rk = __shfl_sync(0xFFFFFFFFu, rk, int((s / 16u) * 8u + unsigned(row % 8)));
-        if (lane == 0) {
-            const unsigned long long i = atomicAdd(cnt, 1ull);
-            o[4 * i] = key;
-            o[4 * i + 1] = blk_off[b] + rk;
-            o[4 * i + 2] = gt.sums[h];
-            o[4 * i + 3] = row;
+            for (unsigned k = 0; k < 16; k++) rk = (16u * q + k == s) ? rank[k] : rk;
+            rk = __shfl_sync(0xFFFFFFFFu, rk, int((s / 16u) * 8u + unsigned(row % 8)));
+            if (lane == 0) {
+                const unsigned long long i = atomicAdd(cnt, 1ull);
+                o[4 * i] = key;
+                o[4 * i + 1] = blk_off[b] + rk;
+                o[4 * i + 2] = gt.sums[h];
+                o[4 * i + 3] = row;
+            }
         }
     }
     if (!ok) atomicOr(err, kErrCorrupt);
@@ -585,29 +644,37 @@ int launch_q3_tma_w(const ColView &kv, const ColView &gv, const ColView &mv, con
                     const StreamCol &s2, const StreamCol &s3, const Pred &pred, const uint32_t *bits, uint64_t nwords,
                     uint64_t lo, uint64_t span, const GTable &gt, uint32_t *hits, unsigned *d_err, cudaStream_t st) {
     QCfg cfg{g_q3.stages, g_q3.stage_bytes};
-    const size_t table = 3ull * 8 * kQSlots, bitmap = 4 * nwords, half = 4 * ((nwords + 1) / 2);
-    const size_t meta = q3_meta_bytes(cfg.stages);
-    const size_t ring = size_t(cfg.stages) * cfg.stage_bytes;
+    const size_t table = 3ull * 8 * kQSlots + W * sizeof(QWarp), bitmap = 4 * nwords, half = 4 * ((nwords + 1) / 2);
+    // The ring takes what the table, the warps' lists and a bitmap in shared
+    // memory leave: the configured stages, shrunk to at least 24 KiB each, or
+    // fewer of them (a stage holds at least one block of all columns, 16 KiB).
     // staged 1: the bitmap in shared memory beside the configured ring when
-    // it fits, else in global memory.  staged 3: split over a 2-CTA cluster,
-    // the ring's stages shrunk to make room (down to 24 KiB).  Both ways of
-    // making room for a large bitmap were measured slower than reading it
-    // from global memory: for a 2^20-key build side a 2 x 25 KiB ring with
-    // the whole bitmap lost more to the shallower pipeline than the probes
-    // gained, and the cluster split (3 x 38 KiB ring, half the bitmap per
-    // CTA) took 242 us at 2^26 fact rows against 198 us, its distributed
-    // shared-memory probes stalling longer than the L2 ones.
-    const auto fit_stage = [&](size_t words_bytes) -> unsigned {
-        if (meta + table + words_bytes >= kQSmemMax) return 0;
-        const size_t room = kQSmemMax - meta - table - words_bytes;
-        const size_t sb = minu(cfg.stage_bytes, room / cfg.stages / 128 * 128);
-        return sb >= 24576 ? unsigned(sb) : 0;
+    // it fits, else in global memory.  staged 3: split over a 2-CTA cluster.
+    // Both ways of making room for a large bitmap were measured slower than
+    // reading it from global memory (before hits were listed, 2^20 keys, 2^26
+    // fact rows): a 2 x 25 KiB ring with the whole bitmap lost more to the
+    // shallower pipeline than the probes gained, and the cluster split took
+    // 242 us against 198 us.
+    const auto fit_ring = [&](size_t words_bytes, unsigned want) -> QCfg {
+        QCfg c = cfg;
+        for (;; c.stages--) {
+            const size_t fixed = q3_meta_bytes(c.stages) + table + words_bytes;
+            if (fixed + 2 * 16384 > kQSmemMax) return QCfg{0, 0};
+            const size_t sb = minu(cfg.stage_bytes, (kQSmemMax - fixed) / c.stages / 128 * 128);
+            if (sb >= minu(want, cfg.stage_bytes)) {
+                c.stage_bytes = unsigned(sb);
+                return c;
+            }
+            if (c.stages == 2) return QCfg{0, 0};
+        }
     };
     int mode = kBmGlobal;
-    if (g_q3.staged == 1 && meta + ring + table + bitmap <= kQSmemMax) mode = kBmShared;
-    else if (g_q3.staged == 3 && fit_stage(half)) mode = kBmCluster;
-    if (mode == kBmCluster) cfg.stage_bytes = fit_stage(half);
-    const size_t shm = meta + size_t(cfg.stages) * cfg.stage_bytes + table +
+    const QCfg rs = fit_ring(bitmap, 40960), rc3 = fit_ring(half, 24576);
+    if (g_q3.staged == 1 && rs.stages == cfg.stages) mode = kBmShared;
+    else if (g_q3.staged == 3 && rc3.stages == cfg.stages) mode = kBmCluster;
+    cfg = mode == kBmShared ? rs : mode == kBmCluster ? rc3 : fit_ring(0, 24576);
+    if (!cfg.stages) return ms_fail(MS_ERR_INVALID, "query3: launch configuration does not fit shared memory");
+    const size_t shm = q3_meta_bytes(cfg.stages) + size_t(cfg.stages) * cfg.stage_bytes + table +
                        (mode == kBmShared ? bitmap : mode == kBmCluster ? half : 0);
     switch (mode) {
     case kBmShared:
@@ -756,7 +823,7 @@ extern "C" int ms_gpu_query3(const ms_col *filter, int cmp, uint64_t c, const ms
             }
             MS_CUDA_TRY(cudaEventRecord(g_q3_ev[1], st));
             MS_CUDA_TRY((scan_exclusive<uint32_t, 1>(hits, nbt, boff, tot, scr, st)));
-            k_q3_extents<<<unsigned(minu(slots / 8, 4096)), 256, 0, st>>>(
+            k_q3_extents<<<unsigned(minu(slots / 256, persistent_grid(256, 2))), 256, 0, st>>>(
                 gt, fv, kv, cmp, c, bits, lo, span, boff, cnt, out, a->d_err);
             MS_CUDA_TRY(cudaGetLastError());
         }
