@@ -68,6 +68,7 @@ _sig = {
     "ms_gpu_arena_used": (C.c_int, [_V, _P(_U64)]),
     "ms_gpu_arena_destroy": (C.c_int, [_V]),
     "ms_gpu_arena_check": (C.c_int, [_V, _V]),
+    "ms_gpu_memcpy": (C.c_int, [_V, _V, _U64, C.c_int, C.c_int, _V]),
     "ms_size_max_byte_any_len": (_U64, [C.c_int, C.c_uint, _U64]),
     "ms_rest_offset": (_U64, [C.c_int, C.c_uint, _U64]),
     "ms_host_build_index": (C.c_int, [C.c_int, _V, _U64, _U64, _V, _V]),
@@ -168,11 +169,17 @@ def _fmt(f) -> Format:
 # ---------------------------------------------------------------------------
 # device memory
 # ---------------------------------------------------------------------------
+_torch_module = None
+
+
 def _torch():
-    import torch  # plumbing only: host<->device copies and streams
-    if not torch.cuda.is_available():
-        raise MorphStoreError(3, "engine_b200 needs a CUDA device")
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch  # plumbing only: host<->device copies and streams
+        if not torch.cuda.is_available():
+            raise MorphStoreError(3, "engine_b200 needs a CUDA device")
+        _torch_module = torch
+    return _torch_module
 
 
 class Arena:
@@ -250,11 +257,20 @@ def _device_view(ptr: int, nbytes: int):
     return torch.as_tensor(_Holder(), device="cuda")
 
 
-def _memcpy_d2h(src: int, nbytes: int) -> np.ndarray:
+_ALL_STREAMS = object()
+
+
+def _memcpy_d2h(src: int, nbytes: int, stream=_ALL_STREAMS) -> np.ndarray:
+    """Device bytes on the host, after all work on the device or, when the
+    stream that wrote them is given, after that stream's."""
+    out = np.empty(nbytes, dtype=np.uint8)
     if nbytes == 0:
-        return np.zeros(0, dtype=np.uint8)
-    _torch().cuda.synchronize()
-    return _device_view(src, nbytes).cpu().numpy().copy()
+        return out
+    if stream is _ALL_STREAMS:
+        _torch().cuda.synchronize()
+        stream = None
+    _check(_lib.ms_gpu_memcpy(out.ctypes.data, src, nbytes, 1, 1, _stream_ptr(stream)), "memcpy")
+    return out
 
 
 # ---------------------------------------------------------------------------
@@ -413,7 +429,7 @@ def agg_sum(col: Column, stream=None) -> int:
     p = col.arena.alloc(8)
     _check(_lib.ms_gpu_agg_sum(C.byref(col.desc), p, col.arena.h, _stream_ptr(stream)), "agg_sum")
     col.arena.check(stream)
-    return int(_memcpy_d2h(p, 8).view(np.uint64)[0])
+    return int(_memcpy_d2h(p, 8, stream).view(np.uint64)[0])
 
 
 def select(cmp: int, col: Column, val: int, out_f: Format = uncompr_f, stream=None) -> Column:
@@ -438,8 +454,8 @@ def select_project_sum(x: Column, cmp: int, c: int, y: Column, want_positions: b
     """Fused select(x cmp c) -> project(y) -> agg_sum.  Returns (sum, count)
     or, with want_positions, (sum, count, positions, values) as numpy."""
     a = x.arena
-    ds = a.alloc(8)
-    dc = a.alloc(8)
+    ds = a.alloc(16)
+    dc = ds + 8
     dp = dv = None
     n = x.get_count_values()
     if want_positions:
@@ -448,11 +464,10 @@ def select_project_sum(x: Column, cmp: int, c: int, y: Column, want_positions: b
     _check(_lib.ms_gpu_select_project_sum(C.byref(x.desc), cmp, c, C.byref(y.desc), ds, dc, dp, dv, a.h,
                                           _stream_ptr(stream)), "select_project_sum")
     a.check(stream)
-    s = int(_memcpy_d2h(ds, 8).view(np.uint64)[0])
-    k = int(_memcpy_d2h(dc, 8).view(np.uint64)[0])
+    s, k = (int(x) for x in _memcpy_d2h(ds, 16, stream).view(np.uint64))
     if not want_positions:
         return s, k
-    return s, k, _memcpy_d2h(dp, 8 * k).view(np.uint64), _memcpy_d2h(dv, 8 * k).view(np.uint64)
+    return s, k, _memcpy_d2h(dp, 8 * k, stream).view(np.uint64), _memcpy_d2h(dv, 8 * k, stream).view(np.uint64)
 
 
 def semi_join(l: Column, r: Column, out_f: Format = uncompr_f, stream=None) -> Column:
@@ -571,8 +586,8 @@ class Batch:
         self.h = _V()
         _check(_lib.ms_gpu_batch_create(descs, cv.ctypes.data if n else None, n, cmp, self.arena.h,
                                         C.byref(self.h), _stream_ptr(stream)), "batch_create")
-        self.d_cnt = self.arena.alloc(8 * max(n, 1))
-        self.d_sum = self.arena.alloc(8 * max(n, 1))
+        self.d_cnt = self.arena.alloc(16 * max(n, 1))
+        self.d_sum = self.d_cnt + 8 * n
 
     def set_config(self, warps: int = 12, stages: int = 2, stage_bytes: int = 8192, ctas_per_sm: int = 1) -> None:
         t = MsTuning(staged=1, warps=warps, stages=stages, stage_bytes=stage_bytes, ctas_per_sm=ctas_per_sm,
@@ -615,9 +630,8 @@ class Batch:
         self.arena.check()
         if not self.n:
             return np.zeros(0, np.uint64), np.zeros(0, np.uint64)
-        cnt = _memcpy_d2h(self.d_cnt, 8 * self.n).view(np.uint64)
-        s = _memcpy_d2h(self.d_sum, 8 * self.n).view(np.uint64)
-        return cnt, s
+        both = _memcpy_d2h(self.d_cnt, 16 * self.n).view(np.uint64)
+        return both[: self.n], both[self.n:]
 
     def run(self, graph: bool = False, stream=None):
         self.launch(graph, stream)

@@ -17,6 +17,7 @@
 #include "delta.cuh"
 #include "fastpath.cuh"
 #include "internal.h"
+#include "readback.cuh"
 #include "rounds.cuh"
 #include "scan.cuh"
 #include "tma.cuh"
@@ -950,9 +951,11 @@ static int encode_rle(const uint64_t *d_in, uint64_t n, ms_col *out, ms_arena *a
         MS_CUDA_TRY(cudaMemsetAsync(words, 0, 4 * (nwords + 2), st));
         int rc = launch_rounds(k_rle_encode, tiles, st, d_in, n, words, (ulonglong2 *)data, d_runs, a->d_err);
         if (rc) return rc;
-        MS_CUDA_TRY(cudaMemcpyAsync(&runs, d_runs, 8, cudaMemcpyDeviceToHost, st));
-        rc = read_err(a, st);  // synchronises the stream
+        ReadBack back(a, st);
+        const uint64_t *h_runs = back.add(d_runs);
+        rc = back.wait();  // synchronises the stream
         if (rc) return rc;
+        runs = *h_runs;
     }
     *out = ms_col{};
     out->format = MS_FMT_RLE;
@@ -1056,9 +1059,11 @@ static int encode(const uint64_t *d_in, uint64_t n, uint64_t ncompr, Layout L, m
                                                                                compr, data);
         MS_CUDA_TRY(cudaGetLastError());
     }
-    if (d_compr) MS_CUDA_TRY(cudaMemcpyAsync(&compr, d_compr, 8, cudaMemcpyDeviceToHost, st));
-    int rc = read_err(a, st);  // synchronises
+    ReadBack back(a, st);
+    const uint64_t *h_compr = d_compr ? back.add(d_compr) : &compr;
+    int rc = back.wait();  // synchronises
     if (rc) return rc;
+    compr = *h_compr;
     *out = ms_col{};
     out->format = uint32_t(fmt);
     out->bw = fmt == MS_FMT_STATIC_VBP ? L.bw : 0;

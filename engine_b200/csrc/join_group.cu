@@ -815,10 +815,11 @@ extern "C" int ms_gpu_semi_join(const ms_col *l, const ms_col *r, int out_format
         MS_CUDA_TRY(cudaMemsetAsync(has_max, 0, 4, st));
         k_build_set<<<grid_blocks(nbl), 256, 0, st>>>(lv, nullptr, 0, slots, s.mask, has_max, a->d_err);
         MS_CUDA_TRY(cudaGetLastError());
-        int hm = 0;
-        MS_CUDA_TRY(cudaMemcpyAsync(&hm, has_max, 4, cudaMemcpyDeviceToHost, st));
-        MS_CUDA_TRY(cudaStreamSynchronize(st));
-        s.has_max = hm;
+        ReadBack back(a, st);
+        const int *hm = back.add(has_max);
+        rc = back.wait_results();
+        if (rc) return rc;
+        s.has_max = *hm;
     }
     const uint64_t words = (s.span + 31) / 32;
     const uint64_t nbt = rv.nblocks_total();
@@ -925,14 +926,15 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
             }
             MS_CUDA_TRY(cudaGetLastError());
         }
-        uint64_t groups = 0;
-        MS_CUDA_TRY(cudaMemcpyAsync(&groups, t.fill, 8, cudaMemcpyDeviceToHost, st));
-        rc = read_err(a, st);
+        ReadBack back(a, st);
+        const unsigned long long *h_groups = back.add(t.fill);
+        rc = back.wait();
         if (rc == MS_ERR_NOMEM && cap < 4 * n + 4096) {
             cap *= 8;  // more distinct keys than the table holds: grow and redo
             continue;
         }
         if (rc) return rc;
+        const uint64_t groups = *h_groups;
         uint64_t *ext = arena_take_t<uint64_t>(a, groups + 1);
         uint64_t *gr = arena_take_t<uint64_t>(a, n + 1);
         if (!ext || !gr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (group output)");
@@ -975,10 +977,11 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
             }
             MS_CUDA_TRY(cudaGetLastError());
         }
-        uint64_t n_scal_groups = 0;
-        MS_CUDA_TRY(cudaMemcpyAsync(&n_scal_groups, words + 2, 8, cudaMemcpyDeviceToHost, st));
-        rc = read_err(a, st);
+        ReadBack end(a, st);
+        const unsigned long long *h_scal = end.add(words + 2);
+        rc = end.wait();
         if (rc) return rc;
+        const uint64_t n_scal_groups = *h_scal;
         const uint64_t n_scal_rows = n - sf;
         rc = write_values(gr, n - n_scal_rows, n_scal_rows, gr_format, 0, out_gr, a, st);
         if (rc) return rc;

@@ -18,10 +18,9 @@
 // 244 us.  Pass 1 is bound by decoding and look-ups, pass 2 by its writes.
 #pragma once
 
-#include <vector>
-
 #include "fastpath.cuh"
 #include "internal.h"
+#include "readback.cuh"
 
 namespace ms {
 namespace {
@@ -209,40 +208,43 @@ int rows_by_mask(const ColView &x, Pass1 pass1, uint64_t **d_pos, uint64_t **d_v
     constexpr bool kBoth = kOut == (kRows | kVals);
     const uint64_t per = 64 + (kOut & kVals ? kBlock * sizeof(V) : 0);  // bytes per block
     TopScratch ts(a);
-    unsigned long long *words = ts.take<unsigned long long>(4);  // running base (two words), remainder hits
-    if (!words) return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions)");
     uint64_t seg = nbt;
     if (per * nbt + (kBoth ? 16 : 8) * n + 4 * kMaxUnits + 4096 > ts.room())
         seg = maxu(1, minu(nbt, 11 * nbt / per));
     const unsigned unit = mask_unit(seg);
-    unsigned *counts = ts.take<unsigned>((seg + unit - 1) / maxu(unit, 1) + 1);
+    const uint64_t ncounts = (seg + unit - 1) / maxu(unit, 1) + 1;
+    // running base (two words), remainder hits; then the units' counts
+    unsigned long long *words = ts.take<unsigned long long>(4 + (ncounts + 1) / 2);
+    unsigned *counts = reinterpret_cast<unsigned *>(words + 4);
     uint32_t *bits = ts.take<uint32_t>(seg * kBlockWords);
     V *side = kOut & kVals ? ts.take<V>(seg * kBlock) : nullptr;
-    if (!counts || !bits || ((kOut & kVals) && !side)) return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions)");
-    MS_CUDA_TRY(cudaMemsetAsync(words, 0, 32, st));
+    if (!words || !bits || ((kOut & kVals) && !side)) return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions)");
+    MS_CUDA_TRY(cudaMemsetAsync(words, 0, 32 + 4 * ncounts, st));
     auto run_of = [&](uint64_t b0) {
         MaskRun r{b0, minu(seg, nbt - b0), unit, 0, bits, counts};
         r.nunits = unsigned((r.nblk + unit - 1) / unit);
         return r;
     };
+    bool clean = true;  // the counts are zero
     auto first = [&](const MaskRun &r) -> int {
-        MS_CUDA_TRY(cudaMemsetAsync(counts, 0, 4 * r.nunits, st));
+        if (!clean) MS_CUDA_TRY(cudaMemsetAsync(counts, 0, 4 * r.nunits, st));
+        clean = false;
         pass1(r, side);
         MS_CUDA_TRY(cudaGetLastError());
         return MS_OK;
     };
     uint64_t cap = 0, total = 0;
     uint64_t *pos = nullptr, *vals = nullptr;
-    std::vector<unsigned> h;
     if (kBoth) {
         for (uint64_t b0 = 0; b0 < nbt; b0 += seg) {
             const MaskRun r = run_of(b0);
             int rc = first(r);
             if (rc) return rc;
-            h.resize(r.nunits);
-            MS_CUDA_TRY(cudaMemcpyAsync(h.data(), counts, 4 * r.nunits, cudaMemcpyDeviceToHost, st));
-            MS_CUDA_TRY(cudaStreamSynchronize(st));
-            for (unsigned c : h) total += c;
+            ReadBack back(a, st);
+            const unsigned *h = back.add(counts, r.nunits);
+            rc = back.wait_results();
+            if (rc) return rc;
+            for (unsigned u = 0; u < r.nunits; u++) total += h[u];
         }
         if (2 * align_up(8 * (total + 1), 256) > ts.room()) return ms_fail(MS_ERR_NOMEM, "arena exhausted (positions output)");
         pos = arena_take_t<uint64_t>(a, total + 1);
@@ -263,9 +265,9 @@ int rows_by_mask(const ColView &x, Pass1 pass1, uint64_t **d_pos, uint64_t **d_v
                                                           side, vals, words + 2);
         MS_CUDA_TRY(cudaGetLastError());
     }
-    unsigned long long hw[3];
-    MS_CUDA_TRY(cudaMemcpyAsync(hw, words, 24, cudaMemcpyDeviceToHost, st));
-    int rc = read_err(a, st);
+    ReadBack back(a, st);
+    const unsigned long long *hw = back.add(words, 3);
+    int rc = back.wait();
     if (rc) return rc;
     if (!kBoth) {
         total = hw[ping];
@@ -330,9 +332,10 @@ inline int key_range(const ColView &c, unsigned long long *words, uint64_t *lo, 
     k_key_range<<<unsigned(maxu(1, minu((nb + 7) / 8, persistent_grid(256, 8)))), 256, 0, st>>>(c, words, words + 1,
                                                                                                 a->d_err);
     MS_CUDA_TRY(cudaGetLastError());
-    unsigned long long h[2];
-    MS_CUDA_TRY(cudaMemcpyAsync(h, words, 16, cudaMemcpyDeviceToHost, st));
-    MS_CUDA_TRY(cudaStreamSynchronize(st));
+    ReadBack back(a, st);
+    const unsigned long long *h = back.add(words, 2);
+    int rc = back.wait_results();
+    if (rc) return rc;
     *lo = h[0];
     *hi = ~h[1];
     return MS_OK;

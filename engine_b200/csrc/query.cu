@@ -781,7 +781,8 @@ extern "C" int ms_gpu_query3(const ms_col *filter, int cmp, uint64_t c, const ms
     // The global group table starts at 2^16 slots and grows by 16x (up to
     // 2^24) when it fills, re-running the pass.
     uint64_t slots = uint64_t(1) << 16;
-    std::vector<uint64_t> rec;  // (key, extent, sum, first row) per group
+    std::vector<uint64_t> more;     // records beyond the first kQFirstGroups
+    const uint64_t *rec = nullptr;  // (key, extent, sum, first row) per group
     uint64_t ng = 0, np = 0;
     for (;;) {
         const uint64_t mark = a->used;
@@ -829,32 +830,33 @@ extern "C" int ms_gpu_query3(const ms_col *filter, int cmp, uint64_t c, const ms
         }
         // counts, error word and the first kQFirstGroups records in one
         // read-back; more groups take a second copy
-        unsigned herr = 0;
-        uint64_t hc[2] = {0, 0};
         const uint64_t first = minu(slots, kQFirstGroups);
-        rec.resize(4 * first);
-        MS_CUDA_TRY(cudaMemcpyAsync(&herr, a->d_err, sizeof herr, cudaMemcpyDeviceToHost, st));
-        MS_CUDA_TRY(cudaMemcpyAsync(hc, cnt, 8, cudaMemcpyDeviceToHost, st));
-        MS_CUDA_TRY(cudaMemcpyAsync(hc + 1, tot, 8, cudaMemcpyDeviceToHost, st));
-        if (nbt) MS_CUDA_TRY(cudaMemcpyAsync(rec.data(), out, 32 * first, cudaMemcpyDeviceToHost, st));
-        MS_CUDA_TRY(cudaStreamSynchronize(st));
-        if (herr == kErrCapacity && slots < (uint64_t(1) << 24)) {
-            MS_CUDA_TRY(cudaMemsetAsync(a->d_err, 0, sizeof herr, st));
+        ReadBack back(a, st);
+        const unsigned *herr = back.add(a->d_err);
+        const unsigned long long *hng = back.add(cnt);
+        const uint64_t *hnp = back.add(tot);
+        if (nbt) rec = back.add(out, 4 * first);
+        rc = back.wait_results();
+        if (rc) return rc;
+        if (*herr == kErrCapacity && slots < (uint64_t(1) << 24)) {
+            MS_CUDA_TRY(cudaMemsetAsync(a->d_err, 0, sizeof *herr, st));
             a->used = mark;
             slots <<= 4;
             continue;
         }
-        rc = read_err(a, st);
+        rc = error_status(*herr, a, st);
         if (rc) return rc;
         float pass_ms = 0;
         if (nbt && cudaEventElapsedTime(&pass_ms, g_q3_ev[0], g_q3_ev[1]) == cudaSuccess) g_q3_pass_ms = pass_ms;
-        ng = hc[0];
-        np = hc[1];
+        ng = *hng;
+        np = *hnp;
         if (ng > first) {
-            rec.resize(4 * ng);
-            MS_CUDA_TRY(cudaMemcpyAsync(rec.data() + 4 * first, out + 4 * first, 32 * (ng - first),
+            more.resize(4 * ng);
+            std::copy(rec, rec + 4 * first, more.begin());
+            MS_CUDA_TRY(cudaMemcpyAsync(more.data() + 4 * first, out + 4 * first, 32 * (ng - first),
                                         cudaMemcpyDeviceToHost, st));
             MS_CUDA_TRY(cudaStreamSynchronize(st));
+            rec = more.data();
         }
         break;
     }

@@ -8,6 +8,7 @@
 
 #include "delta.cuh"
 #include "internal.h"
+#include "readback.cuh"
 
 static thread_local char g_last_error[256];
 
@@ -138,18 +139,33 @@ extern "C" int ms_gpu_stream_sync(void *stream) {
     return MS_OK;
 }
 
-int ms::read_err(ms_arena *a, cudaStream_t st) {
-    unsigned h = 0;
-    MS_CUDA_TRY(cudaMemcpyAsync(&h, a->d_err, sizeof h, cudaMemcpyDeviceToHost, st));
-    MS_CUDA_TRY(cudaStreamSynchronize(st));
-    if (h) {
-        MS_CUDA_TRY(cudaMemsetAsync(a->d_err, 0, sizeof h, st));
-        if (h & kErrCorrupt) return ms_fail(MS_ERR_CORRUPT, "kernel found a corrupt header or bit width");
-        if (h & kErrTimeout) return ms_fail(MS_ERR_TIMEOUT, "bounded device wait gave up");
-        if (h & kErrCapacity) return ms_fail(MS_ERR_NOMEM, "output capacity exceeded on the device");
+namespace {
+
+struct PinnedBuffer {
+    void *p = nullptr;
+    ~PinnedBuffer() {
+        if (p) cudaFreeHost(p);
     }
+};
+
+}  // namespace
+
+void *ms::readback_buffer() {
+    static thread_local PinnedBuffer b;
+    if (!b.p && cudaHostAlloc(&b.p, kReadBackBytes, cudaHostAllocPortable) != cudaSuccess) b.p = nullptr;
+    return b.p;
+}
+
+int ms::error_status(unsigned err, ms_arena *a, cudaStream_t st) {
+    if (!err) return MS_OK;
+    MS_CUDA_TRY(cudaMemsetAsync(a->d_err, 0, sizeof err, st));
+    if (err & kErrCorrupt) return ms_fail(MS_ERR_CORRUPT, "kernel found a corrupt header or bit width");
+    if (err & kErrTimeout) return ms_fail(MS_ERR_TIMEOUT, "bounded device wait gave up");
+    if (err & kErrCapacity) return ms_fail(MS_ERR_NOMEM, "output capacity exceeded on the device");
     return MS_OK;
 }
+
+int ms::read_err(ms_arena *a, cudaStream_t st) { return ReadBack(a, st).wait(); }
 
 extern "C" int ms_gpu_arena_check(ms_arena *a, void *stream) {
     if (!a) return ms_fail(MS_ERR_INVALID, "arena_check: null");
