@@ -23,7 +23,9 @@
 // delta+dvbp = 67, for+dvbp = 69; rle, which the reference's container does
 // not offer, = 71), padding to the next 64-B boundary, then the block's
 // payload.
+#include "fastpath.cuh"
 #include "internal.h"
+#include "readback.cuh"
 #include "scan.cuh"
 
 namespace ms {
@@ -66,74 +68,69 @@ __host__ __device__ inline uint8_t cand_code(const BlockStats &s, unsigned c) {
 
 namespace {
 
-__device__ __forceinline__ uint64_t wor(uint64_t x) {
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) x |= __shfl_xor_sync(0xFFFFFFFFu, x, s);
-    return x;
+__device__ __forceinline__ unsigned warp_width(uint64_t x) {
+    const unsigned hi = __reduce_or_sync(0xFFFFFFFFu, unsigned(x >> 32)), lo = __reduce_or_sync(0xFFFFFFFFu, unsigned(x));
+    return effective_bitwidth(uint64_t(hi) << 32 | lo);
 }
 
-// Analysis of one block by one warp.  Thread `lane` reads rows
-// j = k*32 + lane (k = 0..63): row j belongs to sub-block k/16 and TVL lane
-// j%8 = lane%8.
-// U: unrolling of the four sub-block rounds (4: all 64 loads of a thread in
-// flight; 1: a quarter of the registers, for kernels that want occupancy).
-template <int U = 4>
+// Analysis of one block by one warp, each half of 1024 rows in registers:
+// thread (l, q) holds rows (16q + k) * 8 + l of its sub-blocks, so that the
+// value eight rows before is the thread's previous one and the row before is
+// one shuffle away (l = 0 takes it from l = 7's value eight rows before).  2^26
+// values: 95 us, 82 at the copy rate (171 us with lane-strided rows, eight
+// shuffles per value and a second read for the FOR offsets).
 __device__ BlockStats analyze_block(const uint64_t *__restrict__ x, unsigned lane) {
     BlockStats s;
-    uint64_t prev = 0;       // x[j - 32] of this thread (previous k)
-    uint64_t last_prev = 0;  // x[j - 1] for lane 0: lane 31 of the previous k
+    const unsigned l = lane & 7u, q = lane >> 3;
+    const uint64_t *const mine = x + 128u * q + l;
+    uint64_t last = 0;  // the thread's last value of the sub-block before
     unsigned heads = 0;
-    // minima of the two 1024-halves; widths packed one byte per sub-block
-    // (no register arrays indexed by the loop counter)
-    int64_t mn0 = INT64_MAX, mn1 = INT64_MAX;
-    uint32_t raw_p = 0, dlt_p = 0, fr_p = 0;
-#pragma unroll U
-    for (unsigned i = 0; i < 4; i++) {
-        uint64_t o_raw = 1, o_dlt = 1;
-        int64_t mi = INT64_MAX;
-#pragma unroll
-        for (unsigned kk = 0; kk < 16; kk++) {
-            const unsigned k = i * 16 + kk;
-            const uint64_t v = __ldg(x + k * 32 + lane);
-            // x[j-8]: lane-8 of this k, or lane+24 of the previous k
-            const uint64_t up8 = __shfl_up_sync(0xFFFFFFFFu, v, 8);
-            const uint64_t pk = __shfl_sync(0xFFFFFFFFu, prev, (lane + 24) & 31u);
-            const uint64_t x8 = lane >= 8 ? up8 : (k ? pk : 0);
-            const uint64_t up1 = __shfl_up_sync(0xFFFFFFFFu, v, 1);
-            const uint64_t x1 = lane >= 1 ? up1 : last_prev;
-            heads += (k == 0 && lane == 0) ? 1u : unsigned(v != x1);
-            o_raw |= v;
-            o_dlt |= v - x8;
-            mi = min(mi, (int64_t)v);
-            last_prev = __shfl_sync(0xFFFFFFFFu, v, 31);
-            prev = v;
-        }
-        if (i < 2) mn0 = min(mn0, mi);
-        else mn1 = min(mn1, mi);
-        raw_p |= uint32_t(effective_bitwidth(wor(o_raw))) << (8 * i);
-        dlt_p |= uint32_t(effective_bitwidth(wor(o_dlt))) << (8 * i);
-    }
-    // FOR references: signed minimum per TVL lane, unsigned across lanes
-#pragma unroll
+    uint32_t raw_p = 0, dlt_p = 0, fr_p = 0;  // widths, one byte per sub-block
+#pragma unroll 1
     for (unsigned hh = 0; hh < 2; hh++) {
-        int64_t m = hh ? mn1 : mn0;
-        m = min(m, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (uint64_t)m, 8));
-        m = min(m, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (uint64_t)m, 16));
-        uint64_t um = (uint64_t)m;
+        uint64_t v[32];
+#pragma unroll
+        for (int k = 0; k < 32; k++) v[k] = __ldg(mine + 1024u * hh + 512 * (k >> 4) + 8 * (k & 15));
+        int64_t mn = INT64_MAX;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            uint64_t o_raw = 1, o_dlt = 1;
+            // eight rows before the thread's first: quarter q - 1's last, or
+            // quarter 3's of the sub-block before
+            const uint64_t up = __shfl_up_sync(0xFFFFFFFFu, v[16 * i + 15], 8);
+            const uint64_t wrap = __shfl_sync(0xFFFFFFFFu, last, int(24 + l));
+            uint64_t p = q ? up : wrap;
+            last = v[16 * i + 15];
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                const uint64_t c = v[16 * i + k];
+                const uint64_t before = __shfl_sync(0xFFFFFFFFu, l == 7 ? p : c, int((lane & 24u) | ((l + 7u) & 7u)));
+                // the block's first row starts a run whatever is before it
+                heads += (hh == 0 && i == 0 && k == 0 && lane == 0) ? 1u : unsigned(c != before);
+                o_raw |= c;
+                o_dlt |= c - p;
+                mn = min(mn, (int64_t)c);
+                p = c;
+            }
+            raw_p |= warp_width(o_raw) << (8 * (2 * hh + i));
+            dlt_p |= warp_width(o_dlt) << (8 * (2 * hh + i));
+        }
+        // FOR reference: signed minimum per TVL lane, unsigned across lanes
+        mn = min(mn, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (uint64_t)mn, 8));
+        mn = min(mn, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (uint64_t)mn, 16));
+        uint64_t um = (uint64_t)mn;
         um = minu(um, __shfl_xor_sync(0xFFFFFFFFu, um, 1));
         um = minu(um, __shfl_xor_sync(0xFFFFFFFFu, um, 2));
         um = minu(um, __shfl_xor_sync(0xFFFFFFFFu, um, 4));
         if (um == ~uint64_t(0)) um--;
         s.ref[hh] = um;
-    }
-    // FOR offsets (second read of the block, from L1/L2)
-#pragma unroll U
-    for (unsigned i = 0; i < 4; i++) {
-        uint64_t o = 1;
-        const uint64_t ref = i < 2 ? s.ref[0] : s.ref[1];
 #pragma unroll
-        for (unsigned kk = 0; kk < 16; kk++) o |= __ldg(x + (i * 16 + kk) * 32 + lane) - ref;
-        fr_p |= uint32_t(effective_bitwidth(wor(o))) << (8 * i);
+        for (int i = 0; i < 2; i++) {
+            uint64_t o = 1;
+#pragma unroll
+            for (int k = 0; k < 16; k++) o |= v[16 * i + k] - um;
+            fr_p |= warp_width(o) << (8 * (2 * hh + i));
+        }
     }
 #pragma unroll
     for (unsigned i = 0; i < 4; i++) {
@@ -158,7 +155,7 @@ __device__ __forceinline__ unsigned best_cand(const BlockStats &s) {
     return best;
 }
 
-__global__ void __launch_bounds__(256) k_sel_analyze(const uint64_t *__restrict__ in, uint64_t nblk,
+__global__ void __launch_bounds__(256, 2) k_sel_analyze(const uint64_t *__restrict__ in, uint64_t nblk,
                                                     BlockStats *__restrict__ st, uint32_t *__restrict__ sizes) {
     const unsigned lane = threadIdx.x & 31u;
     for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < nblk;
@@ -185,7 +182,7 @@ __global__ void __launch_bounds__(256, 2) k_sel_resolve(const uint64_t *__restri
         const bool open = mine < nblk && choice[mine] == 255;
         for (unsigned todo = __ballot_sync(0xFFFFFFFFu, open); todo; todo &= todo - 1) {
             const uint64_t b = b0 + uint64_t(__ffs(todo) - 1) * W;
-            const BlockStats s = analyze_block<1>(in + b * kSelBlock, lane);
+            const BlockStats s = analyze_block(in + b * kSelBlock, lane);
             if (lane == 0) choice[b] = uint8_t(best_cand(s));
         }
     }
@@ -564,17 +561,16 @@ extern "C" int ms_gpu_bwi_compress(const uint64_t *d_in, uint64_t nblk, const vo
     k_bwi_sizes<<<sel_grid(nblk), 256, 0, st>>>((const BlockStats *)d_stats, d_choice, nblk, sz);
     MS_CUDA_TRY(cudaGetLastError());
     MS_CUDA_TRY((scan_exclusive<uint64_t, 1>(sz, nblk, off, tot, scr, st)));
-    uint64_t bytes = 0, last_off = 0;
-    uint8_t last_choice = 0;
-    BlockStats last_st{};
+    uint64_t bytes = 0;
     if (nblk) {
-        MS_CUDA_TRY(cudaMemcpyAsync(&last_off, off + nblk - 1, 8, cudaMemcpyDeviceToHost, st));
-        MS_CUDA_TRY(cudaMemcpyAsync(&last_choice, d_choice + nblk - 1, 1, cudaMemcpyDeviceToHost, st));
-        MS_CUDA_TRY(cudaMemcpyAsync(&last_st, (const BlockStats *)d_stats + nblk - 1, sizeof(BlockStats),
-                                    cudaMemcpyDeviceToHost, st));
+        ReadBack back(a, st);
+        const uint64_t *last_off = back.add(off + nblk - 1);
+        const uint8_t *last_choice = back.add(d_choice + nblk - 1);
+        const BlockStats *last_st = back.add((const BlockStats *)d_stats + nblk - 1);
+        int rc = back.wait_results();
+        if (rc) return rc;
+        bytes = *last_off + 64 + cand_size(*last_st, *last_choice);
     }
-    MS_CUDA_TRY(cudaStreamSynchronize(st));
-    if (nblk) bytes = last_off + 64 + cand_size(last_st, last_choice);
     uint8_t *out = arena_take_t<uint8_t>(a, bytes + 64);
     if (!out) return ms_fail(MS_ERR_NOMEM, "arena exhausted (bwi output)");
     if (nblk) {
@@ -655,17 +651,23 @@ __global__ void __launch_bounds__(256) k_sel_gen(uint64_t seed, uint64_t nblk, u
 }
 
 // select(value cmp c) -> sum over a blockwise container.  One warp per
-// block; the four 512-row sub-blocks are decoded with the vbp decoder, the
-// cascade steps applied per format, rle handled per run.
-__global__ void __launch_bounds__(256) k_bwi_select_sum(const uint8_t *__restrict__ data,
-                                                       const uint64_t *__restrict__ q, const uint8_t *__restrict__ codes,
-                                                       const uint32_t *__restrict__ psz, uint64_t nblk, int cmp,
-                                                       uint64_t val,
-                                                       unsigned long long *__restrict__ d_sum,
-                                                       unsigned long long *__restrict__ d_cnt, unsigned *err) {
-    const unsigned lane = threadIdx.x & 31u, l = lane & 7u, qq = lane >> 3;
+// block.  Sub-blocks without a cascade and for_f ones whose values do not
+// cross the signed boundary are selected and summed inside the bit-width switch
+// on 32-bit fields, two at a time (a half-warp each, 32 values per thread);
+// delta and the others are decoded to 64-bit values; rle is handled per run.
+// The header words of the block are read once.  2^26 values of mixed formats:
+// 97 us (226 us with every sub-block decoded to 64-bit values and its header
+// bytes read again).
+__global__ void __launch_bounds__(256, 2) k_bwi_select_sum(const uint8_t *__restrict__ data,
+                                                          const uint64_t *__restrict__ q,
+                                                          const uint8_t *__restrict__ codes,
+                                                          const uint32_t *__restrict__ psz, uint64_t nblk, int cmp,
+                                                          uint64_t val, Pred pred,
+                                                          unsigned long long *__restrict__ d_sum,
+                                                          unsigned long long *__restrict__ d_cnt, unsigned *err) {
+    const unsigned lane = threadIdx.x & 31u, l = lane & 7u, qq = lane >> 3, h = qq & 1u, hb = lane >> 4;
     uint64_t s_sum = 0, s_cnt = 0;
-    bool ok = true;
+    bool ok = true, bad = false;
     for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < nblk;
          b += uint64_t(gridDim.x) * blockDim.x / 32) {
         const unsigned code = codes[b];
@@ -688,62 +690,109 @@ __global__ void __launch_bounds__(256) k_bwi_select_sum(const uint8_t *__restric
             ok &= __reduce_add_sync(0xFFFFFFFFu, unsigned(rows)) == kSelBlock;
             continue;
         }
-        // per sub-block location and width
-        uint64_t carry = 0;  // delta: running lane sum
-        for (unsigned i = 0; i < 4; i++) {
-            unsigned bw;
-            uint64_t off, ref = 0;
-            bool dlt = false;
-            if (code >= 1 && code <= 64) {
-                bw = code;
-                off = uint64_t(64) * bw * i;
-            } else if (code == 65) {
-                uint64_t acc = 0;
-                for (unsigned k = 0; k < i; k++) acc += p[k];
-                bw = p[i];
-                off = 64 + 64 * acc;
-            } else if (code == 67 || code == 69) {
-                const bool isfor = code == 69;
-                const uint64_t page0 = isfor ? 64 : 0;
-                const uint8_t w0 = p[page0], w1 = p[page0 + 1];
-                const uint64_t page1 = page0 + 64 + 64 * uint64_t(w0 + w1);
-                const uint64_t pg = (i >> 1) ? page1 : page0;
-                const uint8_t a = p[pg], c2 = p[pg + 1];
-                bw = (i & 1) ? c2 : a;
-                off = pg + 64 + ((i & 1) ? 64 * uint64_t(a) : 0);
-                if (isfor) ref = reinterpret_cast<const uint64_t *>(p)[i >> 1];
-                else dlt = true;
-            } else {
-                ok = false;
-                break;
+        // widths and offsets of the four sub-blocks, from the header words
+        unsigned bw[4], off[4];
+        uint64_t ref[2] = {0, 0};
+        if (code >= 1 && code <= 64) {
+#pragma unroll
+            for (unsigned i = 0; i < 4; i++) {
+                bw[i] = code;
+                off[i] = 64u * code * i;
             }
-            uint64_t v[16];
-            ok &= vbp_decode16_rt(bw, reinterpret_cast<const uint64_t *>(p + off), l, qq, v);
-            if (dlt) {
+        } else if (code == 65) {
+            const uint64_t w = *reinterpret_cast<const uint64_t *>(p);
+            unsigned at = 64;
+#pragma unroll
+            for (unsigned i = 0; i < 4; i++) {
+                bw[i] = unsigned(w >> (8 * i)) & 0xFFu;
+                off[i] = at;
+                at += 64u * bw[i];
+            }
+        } else if (code == 67 || code == 69) {
+            unsigned pg = 0;
+            if (code == 69) {
+                ref[0] = reinterpret_cast<const uint64_t *>(p)[0];
+                ref[1] = reinterpret_cast<const uint64_t *>(p)[1];
+                pg = 64;
+            }
+#pragma unroll
+            for (unsigned i = 0; i < 2; i++) {
+                const uint64_t w = *reinterpret_cast<const uint64_t *>(p + pg);
+                bw[2 * i] = unsigned(w) & 0xFFu;
+                bw[2 * i + 1] = unsigned(w >> 8) & 0xFFu;
+                off[2 * i] = pg + 64;
+                off[2 * i + 1] = pg + 64 + 64u * bw[2 * i];
+                pg += 64 + 64u * (bw[2 * i] + bw[2 * i + 1]);
+            }
+        } else {
+            ok = false;
+            continue;
+        }
+        if (bw[0] - 1u >= 64u || bw[1] - 1u >= 64u || bw[2] - 1u >= 64u || bw[3] - 1u >= 64u) {
+            ok = false;
+            continue;
+        }
+        if (code == 67) {
+            uint64_t carry = 0;  // running lane sum
+#pragma unroll 1
+            for (unsigned i = 0; i < 4; i++) {
+                const unsigned w = i == 0 ? bw[0] : i == 1 ? bw[1] : i == 2 ? bw[2] : bw[3];
+                const unsigned o = i == 0 ? off[0] : i == 1 ? off[1] : i == 2 ? off[2] : off[3];
+                uint64_t v[16];
+                uint32_t d[16];
+                if (vbp_decode16_u32_rt(w, reinterpret_cast<const uint64_t *>(p + o), l, qq, d)) {
+#pragma unroll
+                    for (int k = 0; k < 16; k++) v[k] = d[k];
+                } else {
+                    ok &= vbp_decode16_rt(w, reinterpret_cast<const uint64_t *>(p + o), l, qq, v);
+                }
 #pragma unroll
                 for (int k = 1; k < 16; k++) v[k] += v[k - 1];
                 const uint64_t tot = v[15];
                 const uint64_t up = __shfl_up_sync(0xFFFFFFFFu, tot, 8);
                 uint64_t pre = qq >= 1 ? up : 0;
                 const uint64_t up2 = __shfl_up_sync(0xFFFFFFFFu, tot + pre, 16);
-                pre += qq >= 2 ? up2 : 0;
-                pre += carry;
+                pre += (qq >= 2 ? up2 : 0) + carry;
 #pragma unroll
-                for (int k = 0; k < 16; k++) v[k] += pre;
+                for (int k = 0; k < 16; k++) {
+                    v[k] += pre;
+                    const bool hit = cmp_eval(cmp, v[k], val, true);
+                    s_sum += hit ? v[k] : 0;
+                    s_cnt += hit;
+                }
                 // lane total of this sub-block: last value of quarter 3
                 carry = __shfl_sync(0xFFFFFFFFu, v[15], 24 + l);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 16; k++) v[k] += ref;
             }
+            continue;
+        }
+#pragma unroll 1
+        for (unsigned i = 0; i < 2; i++) {
+            // sub-block 2i of the first half-warp, 2i + 1 of the second
+            const unsigned w = i ? (hb ? bw[3] : bw[2]) : (hb ? bw[1] : bw[0]);
+            const unsigned o = i ? (hb ? off[3] : off[2]) : (hb ? off[1] : off[0]);
+            const uint64_t *blk = reinterpret_cast<const uint64_t *>(p + o);
+            const uint64_t rf = i ? ref[1] : ref[0];
+            Pred pd = pred;
+            if (code != 69 || (w <= 32 && rel_pred(rf, uint64_t(1) << w, val, cmp, pd))) {
+                unsigned k = 0;
+                const uint64_t t = self_sum32_block_rt(w, blk, l, h, pd, k, bad);
+                s_cnt += k;
+                s_sum += t + uint64_t(k) * rf;
+            } else {
+                for (unsigned part = 2 * h; part < 2 * h + 2; part++) {
+                    uint64_t v[16];
+                    ok &= vbp_decode16_rt(w, blk, l, part, v);
 #pragma unroll
-            for (int k = 0; k < 16; k++)
-                if (cmp_eval(cmp, v[k], val, true)) {
-                    s_sum += v[k];
-                    s_cnt++;
+                    for (int k = 0; k < 16; k++) {
+                        const bool hit = cmp_eval(cmp, v[k] + rf, val, true);
+                        s_sum += hit ? v[k] + rf : 0;
+                        s_cnt += hit;
+                    }
                 }
+            }
         }
     }
+    ok &= !bad;
     if (!ok) atomicOr(err, kErrCorrupt);
     for (int s = 16; s > 0; s >>= 1) {
         s_sum += __shfl_xor_sync(0xFFFFFFFFu, s_sum, s);
@@ -815,7 +864,7 @@ extern "C" int ms_gpu_bwi_select_sum(const uint8_t *d_data, const uint64_t *d_of
     MS_CUDA_TRY(cudaMemsetAsync(d_sum, 0, 8, st));
     if (d_cnt) MS_CUDA_TRY(cudaMemsetAsync(d_cnt, 0, 8, st));
     if (!nblk) return MS_OK;
-    k_bwi_select_sum<<<sel_grid(nblk), 256, 0, st>>>(d_data, d_offsets, d_codes, d_payload_bytes, nblk, cmp, val,
+    k_bwi_select_sum<<<sel_grid(nblk), 256, 0, st>>>(d_data, d_offsets, d_codes, d_payload_bytes, nblk, cmp, val, make_pred(cmp, val),
                                                     (unsigned long long *)d_sum, (unsigned long long *)d_cnt, d_err);
     MS_CUDA_TRY(cudaGetLastError());
     return MS_OK;
