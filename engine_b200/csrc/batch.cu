@@ -37,9 +37,12 @@
 namespace ms {
 namespace {
 
-constexpr unsigned kBItemBlocks = 32;  // blocks per item (one lane each)
+constexpr unsigned kBItemBlocks = 32;  // blocks per item at most (one lane each)
 constexpr unsigned kBItemRest = 4096;  // rows of an uncompressed rest per item
 constexpr unsigned kBItemRuns = 1024;  // runs of an rle_f column per item
+// 32-run pieces of an rle_f item loaded together: one after the other their
+// loads' latency was the tail of the launch (256 columns 135 us -> 119)
+constexpr unsigned kRleAhead = 8;
 
 enum : uint32_t { kItVbp = 0, kItFor = 1, kItDelta = 2, kItRest = 3, kItRle = 4 };
 
@@ -390,24 +393,32 @@ __global__ void __launch_bounds__(32 * W, 1)
             }
         } else {  // rle_f runs, decompressed: rows before sfrom compare signed, the rest unsigned
             const uint64_t *pairs = reinterpret_cast<const uint64_t *>(c.data);
+            const uint64_t end = bi.start + bi.count;
             uint64_t row = bi.seek;
-            for (uint64_t r0 = bi.start; r0 < bi.start + bi.count; r0 += 32) {
-                const uint64_t r = r0 + lane;
-                const bool in = r < bi.start + bi.count;
-                const uint64_t v = in ? __ldg(pairs + 2 * r) : 0, len = in ? __ldg(pairs + 2 * r + 1) : 0;
-                uint64_t incl = len;
+            for (uint64_t r0 = bi.start; r0 < end; r0 += 32 * kRleAhead) {
+                uint64_t v[kRleAhead], len[kRleAhead];
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const uint64_t o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-                    if (int(lane) >= d) incl += o;
+                for (unsigned k = 0; k < kRleAhead; k++) {
+                    const uint64_t r = r0 + 32 * k + lane;
+                    v[k] = r < end ? __ldg(pairs + 2 * r) : 0;
+                    len[k] = r < end ? __ldg(pairs + 2 * r + 1) : 0;
                 }
-                const uint64_t rs = row + incl - len;
-                const uint64_t nsig = c.sfrom > rs ? minu(c.sfrom - rs, len) : 0;
-                const uint64_t add =
-                    (cmp_bits(v, c.c, c.cf, true) ? nsig : 0) + (cmp_bits(v, c.c, c.cf, false) ? len - nsig : 0);
-                cnt += add;
-                sum += v * add;
-                row += __shfl_sync(0xFFFFFFFFu, incl, 31);
+#pragma unroll
+                for (unsigned k = 0; k < kRleAhead; k++) {
+                    uint64_t incl = len[k];
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const uint64_t o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                        if (int(lane) >= d) incl += o;
+                    }
+                    const uint64_t rs = row + incl - len[k];
+                    const uint64_t nsig = c.sfrom > rs ? minu(c.sfrom - rs, len[k]) : 0;
+                    const uint64_t add = (cmp_bits(v[k], c.c, c.cf, true) ? nsig : 0) +
+                                         (cmp_bits(v[k], c.c, c.cf, false) ? len[k] - nsig : 0);
+                    cnt += add;
+                    sum += v[k] * add;
+                    row += __shfl_sync(0xFFFFFFFFu, incl, 31);
+                }
             }
         }
 #pragma unroll
@@ -430,12 +441,12 @@ __global__ void __launch_bounds__(32 * W, 1)
     if (bad && lane == 0) atomicOr(err, kErrCorrupt);
 }
 
-__global__ void k_pick_seeks(const uint64_t *__restrict__ carry, uint64_t nb, uint64_t first_slot,
-                             uint64_t *__restrict__ seeks) {
-    const uint64_t n_it = (nb + kBItemBlocks - 1) / kBItemBlocks;
+__global__ void k_pick_seeks(const uint64_t *__restrict__ carry, uint64_t nb, unsigned per_item,
+                             uint64_t first_slot, uint64_t *__restrict__ seeks) {
+    const uint64_t n_it = (nb + per_item - 1) / per_item;
     for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n_it * 8;
          i += uint64_t(gridDim.x) * blockDim.x)
-        seeks[(first_slot + i / 8) * 8 + i % 8] = carry[(i / 8) * kBItemBlocks * 8 + i % 8];
+        seeks[(first_slot + i / 8) * 8 + i % 8] = carry[(i / 8) * per_item * 8 + i % 8];
 }
 
 // bit width of every column's first block (the decoder its items take)
@@ -613,6 +624,19 @@ void batch_release(ms_batch *b) {
     }
 }
 
+// Blocks per item.  A warp holds its current item and the next one, so with
+// few items the first grab empties the queue and the launch ends on whichever
+// warp drew the slow ones.  The item is halved, down to 8 blocks, until there
+// are 8 items for each of 16 warps per SM.  256 columns (5.6 k items of 32
+// blocks): 225 us with 32 blocks per item, 125 with 16, 118
+// with 8, 142 with 4, where the queue atomics and the per-item setup show.
+// Thousands of columns keep the 32 that their setup is spread over.
+unsigned item_blocks(uint64_t n_blocks) {
+    unsigned ib = kBItemBlocks;
+    while (ib > 8 && n_blocks / ib < 8ull * 16 * sm_count()) ib /= 2;
+    return ib;
+}
+
 int batch_fail(ms_batch *b, int rc) {
     batch_release(b);
     delete b;
@@ -628,6 +652,10 @@ extern "C" int ms_gpu_batch_create(const ms_col *cols, const uint64_t *consts, u
     *out = nullptr;
     cudaStream_t st = (cudaStream_t)stream;
     std::vector<BCol> hc(n_cols);
+    uint64_t n_blocks = 0;
+    for (uint64_t i = 0; i < n_cols; i++)
+        if (cols[i].format != MS_FMT_RLE && cols[i].format != MS_FMT_UNCOMPR) n_blocks += cols[i].count_values / kBlock;
+    const unsigned ib = item_blocks(n_blocks);
     std::vector<BItem> hi;
     std::vector<uint64_t> rle_cols, delta_cols, first_item(n_cols, 0);
     uint64_t n_seek = 0;
@@ -670,13 +698,13 @@ extern "C" int ms_gpu_batch_create(const ms_col *cols, const uint64_t *consts, u
         b.bw = v.bw;
         const uint32_t kind = c.format == MS_FMT_FOR_DVBP ? kItFor : c.format == MS_FMT_DELTA_DVBP ? kItDelta : kItVbp;
         const uint64_t nb = v.nb();
-        for (uint64_t s = 0; s < nb; s += kBItemBlocks)
-            hi.push_back(BItem{uint32_t(i), kind, s, uint32_t(minu(kBItemBlocks, nb - s)), 0,
-                               kind == kItDelta ? n_seek + s / kBItemBlocks : 0});
+        for (uint64_t s = 0; s < nb; s += ib)
+            hi.push_back(BItem{uint32_t(i), kind, s, uint32_t(minu(ib, nb - s)), 0,
+                               kind == kItDelta ? n_seek + s / ib : 0});
         if (kind == kItDelta && nb) {
             delta_cols.push_back(i);
             first_item[i] = n_seek;  // its first seek slot
-            n_seek += (nb + kBItemBlocks - 1) / kBItemBlocks;
+            n_seek += (nb + ib - 1) / ib;
         }
         for (uint64_t r = v.n_compr; r < v.n; r += kBItemRest)
             hi.push_back(BItem{uint32_t(i), kItRest, r, uint32_t(minu(kBItemRest, v.n - r)), 0, 0});
@@ -700,7 +728,7 @@ extern "C" int ms_gpu_batch_create(const ms_col *cols, const uint64_t *consts, u
         ColView v;
         int rc = prepare_view(&cols[i], a, st, &v);
         if (rc) return batch_fail(b, rc);
-        k_pick_seeks<<<64, 256, 0, st>>>(v.carry, v.nb(), first_item[i], b->d_seeks);
+        k_pick_seeks<<<64, 256, 0, st>>>(v.carry, v.nb(), ib, first_item[i], b->d_seeks);
         MS_CUDA_TRY(cudaGetLastError());
         MS_CUDA_TRY(cudaStreamSynchronize(st));
         a->used = mark;

@@ -185,3 +185,40 @@ def test_batch_empty_and_bad_config(ms, arena, orc):
         b.set_config(warps=5)
     cnt, s = b.run()  # the old configuration still works
     assert (int(cnt[0]), int(s[0])) == _expect(orc, v, 100)
+
+
+@pytest.mark.parametrize("blocks", [0, 320_000, 640_000])
+def test_batch_item_sizes(ms, arena, orc, blocks):
+    """Items of 8, 16 and 32 blocks (few, more and many blocks in the plan):
+    columns that end one block before, at and after an item's edge, and rle
+    columns that end around the pieces loaded together."""
+    lengths = [512 * k + d for k, d in ((7, 0), (8, 0), (9, 5), (15, 9), (16, 0), (17, 1), (31, 0), (32, 0), (33, 3),
+                                        (48, 0), (65, 511))]
+    cols, vals, consts = [], [], []
+    for s in range(4):  # static, dynamic, delta, for of every length
+        for i, n in enumerate(lengths):
+            v, bw = _column(orc, KINDS[s], n, 100 * s + i + 1)
+            cols.append(ms.morph(ms.Column.from_numpy(v, arena), _fmt(ms, KINDS[s], bw)))
+            vals.append(v)
+    for runs in (1, 31, 32, 33, 255, 256, 257, 1023, 1024, 1025, 2049):
+        v = np.repeat(orc.uniform_bits(runs, 20, runs) * np.uint64(2) + (np.arange(runs) % 2).astype(np.uint64), 3)
+        cols.append(ms.morph(ms.Column.from_numpy(v, arena), ms.rle_f))
+        vals.append(v)
+    if blocks:  # larger columns, listed again until the plan has that many blocks
+        big = []
+        for s in range(4):
+            v, bw = _column(orc, KINDS[s], (1 << 20) + 77 * s, 900 + s)
+            big.append((ms.morph(ms.Column.from_numpy(v, arena), _fmt(ms, KINDS[s], bw)), v))
+        for k in range(blocks // 2048 + 1):
+            cols.append(big[k % 4][0])
+            vals.append(big[k % 4][1])
+    seen = {}
+    for v in vals:
+        if id(v) not in seen:
+            c = _median(v)
+            seen[id(v)] = (c, _expect(orc, v, c))
+    b = ms.Batch(cols, [seen[id(v)][0] for v in vals])
+    cnt, s = b.run()
+    for i, v in enumerate(vals):
+        assert (int(cnt[i]), int(s[i])) == seen[id(v)][1], (i, len(v), cols[i].format)
+    b.close()
