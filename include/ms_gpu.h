@@ -291,7 +291,8 @@ int ms_gpu_query3(const ms_col *filter, int cmp, uint64_t c, const ms_col *fk, c
  * distributed shared memory -- with the ring's stages shrunk to make room),
  * warps (consumer warps 8, 16 or 24), stages, stage_bytes; other fields
  * ignored.  Rejects a ring that does not fit shared memory with the 48 KiB
- * group table. */
+ * group table.  The launch takes fewer or smaller stages where the consumer
+ * warps' lists of hits need part of the ring's room. */
 int ms_gpu_set_query_tuning(const ms_tuning *t);
 int ms_gpu_get_query_tuning(ms_tuning *t);
 /* Device time (CUDA events around the fact-table pass: the staged kernel and
