@@ -890,8 +890,9 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
     const uint64_t sf = gr_in ? minu(cv.sfrom, gv.sfrom) : cv.sfrom;
     const bool binary = gr_in != nullptr;
     // 2^16 slots hold 2^15 groups; fewer when the column cannot have as many
-    // groups or the arena is short
-    uint64_t cap = 1024;
+    // groups or the arena is short.  A size that was found too small is not
+    // tried again, so the table is filled once per size at most.
+    uint64_t cap = 1024, least = cap;
     while (cap < (uint64_t(1) << 16) && cap < 2 * n) cap <<= 1;
     const uint64_t mark = a->used;
     for (;;) {
@@ -905,7 +906,7 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
         t.mask = cap - 1;
         t.limit = cap / 2;
         if (!t.e || !t.state || !words || (binary && !t.kb)) {
-            if (cap > 1024 && cap <= (uint64_t(1) << 16)) {
+            if (cap > least) {
                 cap >>= 1;
                 continue;
             }
@@ -930,7 +931,8 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
         const unsigned long long *h_groups = back.add(t.fill);
         rc = back.wait();
         if (rc == MS_ERR_NOMEM && cap < 4 * n + 4096) {
-            cap *= 8;  // more distinct keys than the table holds: grow and redo
+            least = 2 * cap;  // more distinct keys than the table holds: grow and redo
+            cap *= 8;
             continue;
         }
         if (rc) return rc;

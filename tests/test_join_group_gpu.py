@@ -214,3 +214,39 @@ def test_intersect_parts(ms, arena, orc, nl, nr, l_gap, r_gap, code):
     for r in (b, b + np.uint64(int(a[-1]) + 1)):
         out = ms.intersect_sorted(_col(ms, arena, orc, a, code), _col(ms, arena, orc, r, code))
         assert np.array_equal(out.to_numpy(), orc.intersect_sorted(a, r))
+
+
+_SHORT_ARENA = """
+import sys
+import numpy as np
+import engine_b200 as ms
+v = (np.arange(6000, dtype=np.uint64) * np.uint64(7919)) % np.uint64(5000)
+g = v % np.uint64(3)
+for kb in (22, 30, 60, 100, 200, 300, 340, 700, 1500):
+    for binary in (False, True):
+        a = ms.Arena((2 if binary else 1) * 8 * len(v) + 512 + (kb << 10))
+        col = ms.Column.from_numpy(v, a)
+        try:
+            gr, ext = ms.group(col, ms.Column.from_numpy(g, a) if binary else None)
+            print(kb, binary, ext.get_count_values(), len(np.unique(gr.to_numpy())))
+        except ms.MorphStoreError as e:
+            print(kb, binary, "status", e.status)
+        a.close()
+"""
+
+
+def test_group_ends_in_a_short_arena(ms):
+    """A table that fills where no larger one fits: out of memory or the right
+    groups, never the same table again (in a process of its own, so that an
+    endless loop fails the test)."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(ms.__file__)))
+    r = subprocess.run([sys.executable, "-c", _SHORT_ARENA], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    lines = [s.split() for s in r.stdout.splitlines()]
+    assert len(lines) == 18
+    for kb, _, *res in lines:
+        assert res == ["status", "4"] or res == ["5000", "5000"], (kb, res)
+    assert lines[0][2] == "status" and lines[-1][2:] == ["5000", "5000"]
