@@ -682,11 +682,19 @@ __global__ void __launch_bounds__(256, 3) k_group_ids(ColView gin, ColView c, Gr
 // row adds its low word, and its high word plus the carry when that is not
 // zero.  Few groups get several copies, one per lane & (copies - 1), so that
 // the lanes of a warp that hit one frequent group do not serialise; an odd
-// copy stride puts a group's copies in different banks.  More groups: one
-// global atomic per row.  2^25 rows, 1000 Zipf(1.1) groups: 0.103 ms
-// (0.726 ms with the lanes of equal groups combined by shuffles first).
+// copy stride puts a group's copies in different banks.  2^25 rows, 1000
+// Zipf(1.1) groups: 0.103 ms (0.726 ms with the lanes of equal groups combined
+// by shuffles first).
 constexpr unsigned kSumCopyBytes = 32768;    // copies are made while they fit this
 constexpr unsigned kSumSmemGroups = 24576;   // 192 KB of sums
+constexpr unsigned kSumSlots = 4096;         // (group + 1, low, high) slots of a CTA beyond that
+
+__device__ __forceinline__ void sum_add(unsigned *s_lo, unsigned *s_hi, unsigned i, uint64_t d) {
+    const unsigned lo = unsigned(d);
+    const unsigned old = lo ? atomicAdd(s_lo + i, lo) : 0u;
+    const unsigned hi = unsigned(d >> 32) + (old + lo < old ? 1u : 0u);
+    if (hi) atomicAdd(s_hi + i, hi);
+}
 
 __global__ void __launch_bounds__(768, 1) k_grouped_sum(ColView gc, ColView dc, uint64_t ngroups, unsigned copies,
                                                        unsigned stride, unsigned long long *__restrict__ out,
@@ -696,7 +704,7 @@ __global__ void __launch_bounds__(768, 1) k_grouped_sum(ColView gc, ColView dc, 
     for (unsigned i = threadIdx.x; i < 2 * copies * stride; i += blockDim.x) sum_smem[i] = 0;
     __syncthreads();
     const unsigned lane = threadIdx.x & 31u, l = lane & 7u, q = lane >> 3;
-    const unsigned mine = copies ? (lane & (copies - 1)) * stride : 0;
+    const unsigned mine = (lane & (copies - 1)) * stride;
     bool ok = true;
     for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < gc.nblocks_total();
          b += uint64_t(gridDim.x) * blockDim.x / 32) {
@@ -711,18 +719,10 @@ __global__ void __launch_bounds__(768, 1) k_grouped_sum(ColView gc, ColView dc, 
                 ok = false;
                 continue;
             }
-            if (copies) {
-                const unsigned i = mine + unsigned(g[k]), lo = unsigned(d[k]);
-                const unsigned old = lo ? atomicAdd(s_lo + i, lo) : 0u;
-                const unsigned hi = unsigned(d[k] >> 32) + (old + lo < old ? 1u : 0u);
-                if (hi) atomicAdd(s_hi + i, hi);
-            } else {
-                atomicAdd(out + g[k], (unsigned long long)d[k]);
-            }
+            sum_add(s_lo, s_hi, mine + unsigned(g[k]), d[k]);
         }
     }
     if (!ok) atomicOr(err, kErrCorrupt);
-    if (!copies) return;
     __syncthreads();
     for (unsigned i = threadIdx.x; i < ngroups; i += blockDim.x) {
         unsigned long long s = 0;
@@ -730,6 +730,70 @@ __global__ void __launch_bounds__(768, 1) k_grouped_sum(ColView gc, ColView dc, 
             s += ((unsigned long long)s_hi[c * stride + i] << 32) + s_lo[c * stride + i];
         if (s) atomicAdd(out + i, s);
     }
+}
+
+// More groups than that: a CTA sums the groups that find one of two slots of
+// its own, first come, first served -- a group of more than a few in 10^4 rows
+// is seen while slots are free -- and adds the other rows to the global
+// sums.  Rows of one group that meet in a warp there (a group that became
+// frequent when the slots were taken) are added up by shuffles first: the
+// global sums take about one add per cycle and address.  2^23 rows, 30000
+// groups, one of them in 90 % of the rows: 86 us a call, even groups 101,
+// Zipf(1.1) 99 (with one global add per row 4840, 101 and 1910; with the equal
+// lanes of every warp combined first 274, 227 and 1130).
+__global__ void __launch_bounds__(256, 3) k_grouped_sum_many(ColView gc, ColView dc, uint64_t ngroups,
+                                                            unsigned long long *__restrict__ out, unsigned *err) {
+    extern __shared__ __align__(16) unsigned sum_smem[];
+    unsigned *const s_tag = sum_smem, *const s_lo = sum_smem + kSumSlots, *const s_hi = sum_smem + 2 * kSumSlots;
+    for (unsigned i = threadIdx.x; i < 3 * kSumSlots; i += blockDim.x) sum_smem[i] = 0;
+    __syncthreads();
+    const unsigned lane = threadIdx.x & 31u, l = lane & 7u, q = lane >> 3;
+    bool ok = true;
+    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; b < gc.nblocks_total();
+         b += uint64_t(gridDim.x) * blockDim.x / 32) {
+        uint64_t g[16], d[16];
+        unsigned vg, vd;
+        ok &= decode_block(gc, b, l, q, g, vg);
+        ok &= decode_block(dc, b, l, q, d, vd);
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            bool left = (vg >> k) & 1u;  // not added yet
+            if (left && g[k] >= ngroups) {
+                ok = false;
+                left = false;
+            }
+            if (left && g[k] < 0xFFFFFFFFull) {
+                const unsigned tag = unsigned(g[k]) + 1u;
+                unsigned h = (unsigned(g[k]) * 0x9E3779B1u) >> 20;  // 12 bits
+#pragma unroll
+                for (int p = 0; p < 2 && left; p++, h ^= 1u) {
+                    unsigned x = *(volatile unsigned *)(s_tag + h);
+                    if (x == 0) x = atomicCAS(s_tag + h, 0u, tag);
+                    if (x == 0 || x == tag) {
+                        sum_add(s_lo, s_hi, h, d[k]);
+                        left = false;
+                    }
+                }
+            }
+            const unsigned rest = __ballot_sync(0xFFFFFFFFu, left);
+            if (!rest) continue;
+            const int lead = __ffs(rest) - 1;
+            const uint64_t lead_g = __shfl_sync(0xFFFFFFFFu, g[k], lead);  // all lanes take part
+            const bool with = left && g[k] == lead_g;
+            if (__popc(__ballot_sync(0xFFFFFFFFu, with)) >= 4) {
+                uint64_t s = with ? d[k] : 0;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+                if (int(lane) == lead) atomicAdd(out + g[k], (unsigned long long)s);
+                left = left && !with;
+            }
+            if (left) atomicAdd(out + g[k], (unsigned long long)d[k]);
+        }
+    }
+    if (!ok) atomicOr(err, kErrCorrupt);
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < kSumSlots; i += blockDim.x)
+        if (s_tag[i]) atomicAdd(out + (s_tag[i] - 1u), ((unsigned long long)s_hi[i] << 32) + s_lo[i]);
 }
 
 }  // namespace
@@ -1007,23 +1071,25 @@ extern "C" int ms_gpu_agg_sum_grouped(const ms_col *gr, const ms_col *data, uint
     MS_CUDA_TRY(cudaMemsetAsync(res, 0, 8 * (n_groups + 1), st));
     const uint64_t nbt = gv.nblocks_total();
     if (nbt && n_groups) {
-        unsigned copies = 0, stride = 0, threads = 256;
         if (n_groups <= kSumSmemGroups) {
-            copies = 1;
-            stride = unsigned(n_groups) | 1u;
+            unsigned copies = 1;
+            const unsigned stride = unsigned(n_groups) | 1u;
             while (copies < 8 && 16ull * copies * stride <= kSumCopyBytes) copies <<= 1;
+            // three CTAs of 256 threads per SM while their sums fit side by
+            // side, else one of 768
+            const size_t smem = 8ull * copies * stride;
+            const bool wide = smem > 72 * 1024;
+            const unsigned threads = wide ? 768 : 256;
+            if (smem > 48 * 1024)
+                MS_CUDA_TRY(cudaFuncSetAttribute(k_grouped_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+            const uint64_t per = threads / 32;
+            const unsigned grid = unsigned(minu((nbt + per - 1) / per, persistent_grid(threads, wide ? 1 : 3)));
+            k_grouped_sum<<<grid, threads, smem, st>>>(gv, dv, n_groups, copies, stride, (unsigned long long *)res,
+                                                       a->d_err);
+        } else {
+            k_grouped_sum_many<<<unsigned(minu((nbt + 7) / 8, persistent_grid(256, 3))), 256, 12 * kSumSlots, st>>>(
+                gv, dv, n_groups, (unsigned long long *)res, a->d_err);
         }
-        // three CTAs of 256 threads per SM while their sums fit side by side,
-        // else one of 768
-        const size_t smem = 8ull * copies * stride;
-        const bool wide = smem > 72 * 1024;
-        if (wide) threads = 768;
-        if (smem > 48 * 1024)
-            MS_CUDA_TRY(cudaFuncSetAttribute(k_grouped_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        const uint64_t per = threads / 32;
-        const unsigned grid = unsigned(minu((nbt + per - 1) / per, persistent_grid(threads, wide ? 1 : 3)));
-        k_grouped_sum<<<grid, threads, smem, st>>>(gv, dv, n_groups, copies, stride, (unsigned long long *)res,
-                                                   a->d_err);
         MS_CUDA_TRY(cudaGetLastError());
     }
     rc = read_err(a, st);
