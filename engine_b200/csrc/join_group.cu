@@ -802,6 +802,14 @@ static unsigned grid_blocks(uint64_t nbt) {
     return (unsigned)maxu(1, minu((nbt + 7) / 8, persistent_grid(256, 8)));
 }
 
+// Dynamic shared memory that a kernel may be launched with.  The limit belongs to
+// the function, not to a launch, so it is always the kernel's largest: one
+// thread's smaller size would fail another thread's launch.
+template <class... P> static int allow_smem(void (*kern)(P...), unsigned most) {
+    MS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)));
+    return MS_OK;
+}
+
 // The bitmap goes to shared memory when it fits and the probe side is long
 // enough to pay for each SM's copy: an SM copies `words` and then looks up
 // its share of the rows, one word each.
@@ -888,8 +896,10 @@ extern "C" int ms_gpu_semi_join(const ms_col *l, const ms_col *r, int out_format
     const uint64_t words = (s.span + 31) / 32;
     const uint64_t nbt = rv.nblocks_total();
     const bool smem = s.bits && smem_bitmap(words, nbt);
-    if (smem)
-        MS_CUDA_TRY(cudaFuncSetAttribute(k_probe_bits<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(4 * words)));
+    if (smem) {
+        rc = allow_smem(k_probe_bits<true>, 4 * kSmemBitmapWords);
+        if (rc) return rc;
+    }
     auto pass1 = [&](const MaskRun &run, uint32_t *) {
         if (smem)
             k_probe_bits<true><<<mask_grid(run.nblk, kProbeWarps, 1), 32 * kProbeWarps, 4 * words, st>>>(rv, s, run,
@@ -1080,8 +1090,8 @@ extern "C" int ms_gpu_agg_sum_grouped(const ms_col *gr, const ms_col *data, uint
             const size_t smem = 8ull * copies * stride;
             const bool wide = smem > 72 * 1024;
             const unsigned threads = wide ? 768 : 256;
-            if (smem > 48 * 1024)
-                MS_CUDA_TRY(cudaFuncSetAttribute(k_grouped_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+            rc = allow_smem(k_grouped_sum, 8 * (kSumSmemGroups + 1));
+            if (rc) return rc;
             const uint64_t per = threads / 32;
             const unsigned grid = unsigned(minu((nbt + per - 1) / per, persistent_grid(threads, wide ? 1 : 3)));
             k_grouped_sum<<<grid, threads, smem, st>>>(gv, dv, n_groups, copies, stride, (unsigned long long *)res,
@@ -1157,9 +1167,10 @@ extern "C" int ms_gpu_natural_join(const ms_col *l, const ms_col *r, int out_l_f
     // build positions of 32 bits unless the build side is longer
     auto join = [&](auto pos_type) -> int {
         using V = decltype(pos_type);
-        if (smem)
-            MS_CUDA_TRY(cudaFuncSetAttribute(k_probe_map_bits<true, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(4 * words)));
+        if (smem) {
+            int e = allow_smem(k_probe_map_bits<true, V>, 4 * kSmemBitmapWords);
+            if (e) return e;
+        }
         auto pass1 = [&](const MaskRun &run, V *side) {
             if (smem)
                 k_probe_map_bits<true, V><<<mask_grid(run.nblk, kProbeWarps, 1), 32 * kProbeWarps, 4 * words, st>>>(

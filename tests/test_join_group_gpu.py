@@ -300,3 +300,47 @@ def test_grouped_sum_of_a_frequent_group_is_not_serial(ms, arena, orc):
             times.append(time.perf_counter() - t0)
         best.append(min(times))
     assert best[1] < 5 * best[0], best
+
+
+@pytest.mark.parametrize("op", ["agg_sum_grouped", "semi_join", "natural_join"])
+def test_two_threads_with_tables_of_different_sizes(ms, orc, op):
+    """Two host threads, each with its own arena and stream, whose calls need
+    different amounts of shared memory."""
+    import threading
+    import torch
+    n = 1 << 21
+    failed = []
+
+    def calls(size, seed):
+        try:
+            a = ms.Arena(256 << 20)
+            st = torch.cuda.Stream()
+            probe = ms.Column.from_numpy(orc.uniform_bits(seed, 40, n) % np.uint64(size), a)
+            keys = ms.Column.from_numpy(np.array([0, size - 1], np.uint64), a)
+            torch.cuda.synchronize()
+            start.wait()
+            for _ in range(400):
+                probe.arena = keys.arena = scratch[size]  # for results, which are dropped
+                scratch[size].reset()
+                if op == "agg_sum_grouped":
+                    ms.agg_sum_grouped(probe, probe, size, stream=st)
+                elif op == "semi_join":
+                    ms.semi_join(keys, probe, stream=st)
+                else:
+                    ms.natural_join(keys, probe, stream=st)
+            a.close()
+        except Exception as e:  # reported by the main thread
+            failed.append(e)
+
+    # sums of 160 and 56 KB, bitmaps of 50 KB and 250 bytes
+    sizes = (20_000, 7_000) if op == "agg_sum_grouped" else (400_000, 2_000)
+    scratch = {s: ms.Arena(64 << 20) for s in sizes}
+    start = threading.Barrier(len(sizes))
+    threads = [threading.Thread(target=calls, args=(s, i + 1)) for i, s in enumerate(sizes)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for s in scratch.values():
+        s.close()
+    assert not failed, failed
