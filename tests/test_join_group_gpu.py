@@ -344,3 +344,76 @@ def test_two_threads_with_tables_of_different_sizes(ms, orc, op):
     for s in scratch.values():
         s.close()
     assert not failed, failed
+
+
+def _short_of_room(ms, orc, op, n, hits):
+    """The operator's inputs, the bytes they take in an arena, the call and
+    its result: `hits` of n rows hit."""
+    v = np.arange(n, dtype=np.uint64) * np.uint64(3)
+    k = v[:: n // hits][:hits].copy()
+    pos = (np.arange(hits) * (n // hits)).astype(np.uint64)
+    if op == "select":
+        return (v,), lambda c: (ms.select(O.CMP_LT, c, int(v[hits])),), (np.arange(hits, dtype=np.uint64),)
+    if op == "semi_join":
+        return (k, v), lambda l, r: (ms.semi_join(l, r),), (pos,)
+    if op == "natural_join":
+        return (k, v), lambda l, r: ms.natural_join(l, r), (np.arange(hits, dtype=np.uint64), pos)
+    return (v, k), lambda l, r: (ms.intersect_sorted(l, r),), (k,)
+
+
+@pytest.mark.parametrize("op", ["select", "semi_join", "natural_join", "intersect_sorted"])
+@pytest.mark.parametrize("n,hits", [(700, 500), (70_003, 70), (70_003, 60_000)])
+def test_positions_with_every_amount_of_room(ms, orc, op, n, hits):
+    """From no room to plenty: out of memory, then the right result in more
+    and more blocks at once, and never out of memory again."""
+    args, call, want = _short_of_room(ms, orc, op, n, hits)
+    fixed = sum(8 * len(x) + 512 for x in args)
+    a = ms.Arena(fixed + (16 << 20))
+    cols = [ms.Column.from_numpy(x, a) for x in args]
+    seen = []
+    for room in [0] + [int(1.13 ** i) for i in range(50, 130)] + [15 << 20]:
+        left = a.alloc((a.capacity - a.used()) // 256 * 256 - 256 - room // 256 * 256)
+        assert left
+        try:
+            out = call(*cols)
+            seen.append(True)
+            for c, w in zip(out, want):
+                assert np.array_equal(c.to_numpy(), w), room
+        except ms.MorphStoreError as e:
+            assert e.status == 4
+            seen.append(False)
+        a.reset()
+        cols = [ms.Column.from_numpy(x, a) for x in args]
+    assert not seen[0] and seen[-1] and seen == sorted(seen)
+    a.close()
+
+
+@pytest.mark.parametrize("op", ["select", "semi_join", "natural_join", "intersect_sorted"])
+def test_positions_of_few_hits_in_a_short_arena(ms, orc, op):
+    """With room for the bits of all rows (and the values beside them) and for
+    the result, but not for a result of every row, the call takes no longer
+    than in a large arena (intersect_sorted and natural_join went through 380
+    and 190 segments)."""
+    import time
+    import torch
+    n, hits = 1 << 21, 100
+    args, call, want = _short_of_room(ms, orc, op, n, hits)
+    fixed = sum(8 * len(x) + 512 for x in args)
+    per_block = {"select": 64, "semi_join": 64, "natural_join": 64 + 2048, "intersect_sorted": 64 + 4096}[op]
+    tables = (1 << 20) + 5 * 3 * n if op == "natural_join" else (1 << 20)
+    best = []
+    for room in (per_block * (n // 512) + tables, 40 * n + (64 << 20)):
+        a = ms.Arena(fixed + room)
+        times = []
+        for _ in range(8):
+            a.reset()
+            cols = [ms.Column.from_numpy(x, a) for x in args]
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            out = call(*cols)
+            times.append(time.perf_counter() - t0)
+        for c, w in zip(out, want):
+            assert np.array_equal(c.to_numpy(), w)
+        best.append(min(times))
+        a.close()
+    assert best[0] < 3 * best[1], best
