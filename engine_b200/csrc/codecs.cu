@@ -512,8 +512,10 @@ __global__ void __launch_bounds__(kRdThreads, 1)
                 if (tp == ntiles - 1 && w == kRdWarps - 1 && lane == 0) {
                     // the final run ends at row n
                     const uint64_t total = run0 + tot;
+                    uint64_t slot;
                     *d_runs = total;
-                    out[total - 1] = make_ulonglong2(v[n - row0 - 1], n + 1 - (tail ? row0 + tail : pre.last));
+                    if (rle_last_slot(total, n, slot))
+                        out[slot] = make_ulonglong2(v[n - row0 - 1], n + 1 - (tail ? row0 + tail : pre.last));
                 }
             }
             pre.next();

@@ -86,6 +86,14 @@ __host__ __device__ inline uint64_t scalar_from(const ms_col &c) {
     return c.count_values - nrest % kStep;
 }
 
+// Place of an rle column's last pair among the pairs of n rows, `total` being
+// the runs counted.  False when there is none: after a wait that gave up, the
+// counts of earlier tiles may be missing, down to no run at all.
+__host__ __device__ inline bool rle_last_slot(uint64_t total, uint64_t n, uint64_t &slot) {
+    slot = total - 1;
+    return slot < n;
+}
+
 // Bounded spin: iterations before a device-side wait gives up.
 constexpr unsigned kSpinLimit = 1u << 22;
 

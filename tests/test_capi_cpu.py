@@ -77,3 +77,20 @@ def test_col_load_reports_missing_file(tmp_path):
                               None)
     assert rc == 7
     assert b"could not open" in ms.lib().ms_gpu_status_string(rc)
+
+
+def test_rle_last_pair_stays_in_the_output(tmp_path):
+    """The encoder's last pair when counts of earlier tiles are missing (a wait
+    gave up): no run counted gives no place, never one before the output."""
+    import subprocess
+    src = tmp_path / "slot.cpp"
+    src.write_text(f'#include "{ROOT}/engine_b200/csrc/ms_common.cuh"\n'
+                   "#include <stdio.h>\n"
+                   "int main() { uint64_t at;\n"
+                   "  for (uint64_t n : {1ull, 6145ull}) for (uint64_t total : {0ull, 1ull, 2ull, 6145ull, 6146ull})\n"
+                   '    if (ms::rle_last_slot(total, n, at)) printf("%llu:%llu ", (unsigned long long)total, (unsigned long long)at);\n'
+                   '    else printf("%llu:- ", (unsigned long long)total); }\n')
+    exe = tmp_path / "slot"
+    subprocess.run(["g++", "-std=c++17", "-I/usr/local/cuda/include", str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split()
+    assert out == ["0:-", "1:0", "2:-", "6145:-", "6146:-", "0:-", "1:0", "2:1", "6145:6144", "6146:-"]
