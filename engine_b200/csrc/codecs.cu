@@ -12,6 +12,7 @@
 // The same encoder writes operator outputs with the write iterator's
 // 2048-value chunking (write_iterator.h:67-306): only the number of blocks
 // per page changes (64 -> 4 for dynamic_vbp, 8 -> 2 for for_f).
+#include <cuda.h>
 #include <string.h>
 
 #include "delta.cuh"
@@ -923,7 +924,50 @@ __global__ void __launch_bounds__(kRleLbThreads, 2) k_rle_expand_lb(const uint64
 // ---------------------------------------------------------------------------
 // host drivers
 // ---------------------------------------------------------------------------
-// Launch of a rounds kernel: one CTA per SM at most, all resident.
+namespace {
+
+// Driver functions for the partition of the device that a launch runs on.
+struct Partition {
+    CUresult (*current)(CUcontext *) = nullptr;
+    CUresult (*of_ctx)(CUcontext, CUdevResource *, CUdevResourceType) = nullptr;
+    CUresult (*green)(CUstream, CUgreenCtx *) = nullptr;
+    CUresult (*of_green)(CUgreenCtx, CUdevResource *, CUdevResourceType) = nullptr;
+    Partition() {
+        get("cuCtxGetCurrent", current);
+        get("cuCtxGetDevResource", of_ctx);
+        get("cuStreamGetGreenCtx", green);
+        get("cuGreenCtxGetDevResource", of_green);
+    }
+    template <class F> static void get(const char *name, F &f) {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            f = reinterpret_cast<F>(p);
+    }
+};
+
+}  // namespace
+
+// SMs that a launch on `st` gets: those of the stream's or the current green
+// context, else all.
+static unsigned launch_sms(cudaStream_t st) {
+    static const Partition d;
+    unsigned sms = unsigned(sm_count());
+    CUdevResource r;
+    CUcontext ctx = nullptr;
+    if (d.current && d.of_ctx && d.current(&ctx) == CUDA_SUCCESS && ctx &&
+        d.of_ctx(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS)
+        sms = unsigned(minu(sms, r.sm.smCount));
+    CUgreenCtx g = nullptr;
+    const bool own = st && st != cudaStreamLegacy && st != cudaStreamPerThread;
+    if (own && d.green && d.of_green && d.green(st, &g) == CUDA_SUCCESS && g &&
+        d.of_green(g, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS)
+        sms = unsigned(minu(sms, r.sm.smCount));
+    return unsigned(maxu(sms, 1));
+}
+
+// Launch of a rounds kernel: one CTA per SM at most, all resident (the kernels
+// take any number of CTAs).
 template <class... P, class... A>
 static int launch_rounds(void (*kern)(P...), uint64_t ntiles, cudaStream_t st, A... args) {
     constexpr size_t smem = kRdSmem;
@@ -932,7 +976,7 @@ static int launch_rounds(void (*kern)(P...), uint64_t ntiles, cudaStream_t st, A
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
-    lc.gridDim = dim3(unsigned(minu(ntiles, uint64_t(sm_count()))));
+    lc.gridDim = dim3(unsigned(minu(ntiles, launch_sms(st))));
     lc.blockDim = dim3(kRdThreads);
     lc.dynamicSmemBytes = smem;
     lc.stream = st;

@@ -275,3 +275,36 @@ def test_delta_segments(ms, arena, orc, bits, n):
     assert ms.agg_sum(c) == orc.agg_sum(v)
     lanes = v[: n // 1024 * 1024].reshape(-1, 8)[-1]
     assert np.array_equal(c.delta_lane_sums(), lanes)
+
+
+@pytest.mark.parametrize("fmt", [O.DYNAMIC_VBP, O.DELTA_DVBP, O.FOR_DVBP, O.RLE])
+def test_encoders_on_a_part_of_the_sms(ms, arena, orc, fmt):
+    """A stream of a green context of 16 SMs: the encoders' CTAs, which wait on
+    one another, are as many as that partition holds."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        assert r[0] == driver.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+
+    import torch
+    torch.zeros(1, device="cuda")
+    dev = ok(driver.cuDeviceGet(0))
+    sms = ok(driver.cuDeviceGetDevResource(dev, driver.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    part = ok(driver.cuDevSmResourceSplitByCount(1, sms, 0, 16))[0]
+    desc = ok(driver.cuDevResourceGenerateDesc(part[:1], 1))
+    green = ok(driver.cuGreenCtxCreate(desc, dev, driver.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    stream = ok(driver.cuGreenCtxStreamCreate(green, driver.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    try:
+        n = 3 * 148 * 6144 + 1031
+        v = orc.runs(3, 3, 20, n) if fmt == O.RLE else _all_widths(orc, n, 3)
+        col = ms.Column.from_numpy(v, arena)
+        torch.cuda.synchronize()
+        c = ms.morph(col, _fmt(ms, fmt, 0), stream=int(stream))
+        b, m = orc.compress(fmt, 0, v)
+        assert c.meta() == m
+        assert np.array_equal(_masked(fmt, 0, c.raw_bytes(), m, orc), _masked(fmt, 0, b[: m[1]], m, orc))
+    finally:
+        torch.cuda.synchronize()
+        assert driver.cuStreamDestroy(stream)[0] == driver.CUresult.CUDA_SUCCESS
+        assert driver.cuGreenCtxDestroy(green)[0] == driver.CUresult.CUDA_SUCCESS
