@@ -27,7 +27,7 @@
 // fixed sequence of stream operations (three memsets and one launch) with no
 // host synchronisation, so it can be captured into a CUDA graph; the plan
 // keeps one graph per pair of output buffers.
-#include <algorithm>
+#include <memory>
 #include <vector>
 
 #include "fastpath.cuh"
@@ -643,22 +643,16 @@ int batch_fail(ms_batch *b, int rc) {
     return rc;
 }
 
-}  // namespace
-
-extern "C" int ms_gpu_batch_create(const ms_col *cols, const uint64_t *consts, uint64_t n_cols, int cmp, ms_arena *a,
-                                   ms_batch **out, void *stream) {
-    if (!out || !a || (n_cols && (!cols || !consts))) return ms_fail(MS_ERR_INVALID, "batch_create: null argument");
-    if (cmp < MS_CMP_EQ || cmp > MS_CMP_GE) return ms_fail(MS_ERR_INVALID, "batch_create: comparison");
-    *out = nullptr;
-    cudaStream_t st = (cudaStream_t)stream;
+// The plan with `ib` blocks per item.
+int plan_batch(const ms_col *cols, const uint64_t *consts, uint64_t n_cols, int cmp, unsigned ib, ms_arena *a,
+               ms_batch **out, cudaStream_t st) {
     std::vector<BCol> hc(n_cols);
-    uint64_t n_blocks = 0;
-    for (uint64_t i = 0; i < n_cols; i++)
-        if (cols[i].format != MS_FMT_RLE && cols[i].format != MS_FMT_UNCOMPR) n_blocks += cols[i].count_values / kBlock;
-    const unsigned ib = item_blocks(n_blocks);
-    std::vector<BItem> hi;
-    std::vector<uint64_t> rle_cols, delta_cols, first_item(n_cols, 0);
-    uint64_t n_seek = 0;
+    std::vector<uint32_t> kinds(n_cols, kItVbp);
+    std::vector<uint64_t> parts(n_cols, 0);  // blocks of the column, or runs (kItRle)
+    // delta_f: first seek slot; rle_f: first entry of run_rows
+    std::vector<uint64_t> rle_cols, delta_cols, first(n_cols, 0);
+    uint64_t n_items = 0, n_seek = 0, n_rle = 0;
+    const auto pieces = [](uint64_t n, uint64_t per) { return (n + per - 1) / per; };
     for (uint64_t i = 0; i < n_cols; i++) {
         const ms_col &c = cols[i];
         int rc = check_col(&c, false);
@@ -670,11 +664,13 @@ extern "C" int ms_gpu_batch_create(const ms_col *cols, const uint64_t *consts, u
         b.n = c.count_values;
         if (c.format == MS_FMT_RLE) {
             b.data = (const uint8_t *)c.data;
+            b.n_compr = b.n;
             b.sfrom = c.count_values - c.count_values % kStep;  // as the decompressed column
-            const uint64_t runs = c.size_used_byte / 16;
-            first_item[i] = hi.size();
-            for (uint64_t r = 0; r < runs; r += kBItemRuns)
-                hi.push_back(BItem{uint32_t(i), kItRle, r, uint32_t(minu(kBItemRuns, runs - r)), 0, 0});
+            kinds[i] = kItRle;
+            parts[i] = c.size_used_byte / 16;
+            first[i] = n_rle;
+            n_rle += pieces(parts[i], kBItemRuns);
+            n_items += pieces(parts[i], kBItemRuns);
             rle_cols.push_back(i);
             hc[i] = b;
             continue;
@@ -696,68 +692,61 @@ extern "C" int ms_gpu_batch_create(const ms_col *cols, const uint64_t *consts, u
         b.n_compr = v.n_compr;
         b.sfrom = v.sfrom;
         b.bw = v.bw;
-        const uint32_t kind = c.format == MS_FMT_FOR_DVBP ? kItFor : c.format == MS_FMT_DELTA_DVBP ? kItDelta : kItVbp;
-        const uint64_t nb = v.nb();
-        for (uint64_t s = 0; s < nb; s += ib)
-            hi.push_back(BItem{uint32_t(i), kind, s, uint32_t(minu(ib, nb - s)), 0,
-                               kind == kItDelta ? n_seek + s / ib : 0});
-        if (kind == kItDelta && nb) {
+        kinds[i] = c.format == MS_FMT_FOR_DVBP ? kItFor : c.format == MS_FMT_DELTA_DVBP ? kItDelta : kItVbp;
+        parts[i] = v.nb();
+        if (kinds[i] == kItDelta && parts[i]) {
             delta_cols.push_back(i);
-            first_item[i] = n_seek;  // its first seek slot
-            n_seek += (nb + ib - 1) / ib;
+            first[i] = n_seek;
+            n_seek += pieces(parts[i], ib);
         }
-        for (uint64_t r = v.n_compr; r < v.n; r += kBItemRest)
-            hi.push_back(BItem{uint32_t(i), kItRest, r, uint32_t(minu(kBItemRest, v.n - r)), 0, 0});
+        n_items += pieces(parts[i], ib) + pieces(v.n - v.n_compr, kBItemRest);
         hc[i] = b;
     }
     ms_batch *b = new ms_batch{};
     b->arena = a;
     b->n_cols = n_cols;
-    b->n_items = hi.size();
+    b->n_items = n_items;
     b->cfg = ms_tuning{1, 12, 2, 8192, 1, 16};
     b->d_cols = arena_take_t<BCol>(a, n_cols + 1);
-    b->d_items = arena_take_t<BItem>(a, hi.size() + 1);
+    b->d_items = arena_take_t<BItem>(a, n_items + 1);
     b->d_seeks = arena_take_t<uint64_t>(a, 8 * n_seek + 8);
     b->d_head = arena_take_t<unsigned long long>(a, kBatchKinds);
     if (!b->d_cols || !b->d_items || !b->d_seeks || !b->d_head)
         return batch_fail(b, ms_fail(MS_ERR_NOMEM, "arena exhausted (batch plan)"));
-    b->plan_bytes = sizeof(BCol) * n_cols + sizeof(BItem) * hi.size() + 64 * n_seek;
+    b->plan_bytes = sizeof(BCol) * n_cols + sizeof(BItem) * n_items + 64 * n_seek;
     // delta_f seeks: the carry into each item's first block
     for (uint64_t i : delta_cols) {
         const uint64_t mark = a->used;
         ColView v;
         int rc = prepare_view(&cols[i], a, st, &v);
         if (rc) return batch_fail(b, rc);
-        k_pick_seeks<<<64, 256, 0, st>>>(v.carry, v.nb(), ib, first_item[i], b->d_seeks);
+        k_pick_seeks<<<64, 256, 0, st>>>(v.carry, v.nb(), ib, first[i], b->d_seeks);
         MS_CUDA_TRY(cudaGetLastError());
         MS_CUDA_TRY(cudaStreamSynchronize(st));
         a->used = mark;
     }
     // rle_f: the first row of every item
+    std::vector<uint64_t> run_rows(n_rle);
     for (uint64_t i : rle_cols) {
-        const uint64_t runs = cols[i].size_used_byte / 16;
-        const uint64_t n_it = (runs + kBItemRuns - 1) / kBItemRuns;
+        const uint64_t n_it = pieces(parts[i], kBItemRuns);
         if (!n_it) continue;
         const uint64_t mark = a->used;
         uint64_t *tot = arena_take_t<uint64_t>(a, n_it);
         if (!tot) return batch_fail(b, ms_fail(MS_ERR_NOMEM, "arena exhausted (batch plan)"));
-        k_rle_item_rows<<<64, 256, 0, st>>>((const uint64_t *)cols[i].data, runs, tot);
+        k_rle_item_rows<<<64, 256, 0, st>>>((const uint64_t *)cols[i].data, parts[i], tot);
         MS_CUDA_TRY(cudaGetLastError());
-        std::vector<uint64_t> h(n_it);
-        MS_CUDA_TRY(cudaMemcpyAsync(h.data(), tot, 8 * n_it, cudaMemcpyDeviceToHost, st));
+        uint64_t *const h = run_rows.data() + first[i];
+        MS_CUDA_TRY(cudaMemcpyAsync(h, tot, 8 * n_it, cudaMemcpyDeviceToHost, st));
         MS_CUDA_TRY(cudaStreamSynchronize(st));
         a->used = mark;
-        uint64_t row = 0;
-        for (uint64_t k = 0; k < n_it; k++) {
-            hi[first_item[i] + k].seek = row;
-            row += h[k];
+        for (uint64_t k = 0, row = 0; k < n_it; k++) {
+            const uint64_t rows = h[k];
+            h[k] = row;
+            row += rows;
         }
     }
-    if (n_cols) MS_CUDA_TRY(cudaMemcpyAsync(b->d_cols, hc.data(), sizeof(BCol) * n_cols, cudaMemcpyHostToDevice, st));
-    // Queue order: items that take the same decoder (kind, bit width) run
-    // together, so the warps of an SM share their instructions; the items of
-    // a column keep their order.
     if (n_cols) {
+        MS_CUDA_TRY(cudaMemcpyAsync(b->d_cols, hc.data(), sizeof(BCol) * n_cols, cudaMemcpyHostToDevice, st));
         const uint64_t mark = a->used;
         uint8_t *d_bw = arena_take_t<uint8_t>(a, n_cols);
         if (!d_bw) return batch_fail(b, ms_fail(MS_ERR_NOMEM, "arena exhausted (batch plan)"));
@@ -767,26 +756,61 @@ extern "C" int ms_gpu_batch_create(const ms_col *cols, const uint64_t *consts, u
         MS_CUDA_TRY(cudaMemcpyAsync(fbw.data(), d_bw, n_cols, cudaMemcpyDeviceToHost, st));
         MS_CUDA_TRY(cudaStreamSynchronize(st));
         a->used = mark;
-        std::stable_sort(hi.begin(), hi.end(), [&](const BItem &x, const BItem &y) {
-            const uint32_t kx = (x.kind << 8) | (x.kind <= kItDelta ? fbw[x.col] : 0u);
-            const uint32_t ky = (y.kind << 8) | (y.kind <= kItDelta ? fbw[y.col] : 0u);
-            return kx < ky;
-        });
+        // Queue order: items that take the same decoder (kind, bit width) run
+        // together, so the warps of an SM share their instructions; the items
+        // of a column keep their order.  Places are counted, then every item
+        // is written once (sorting the items took 1 ms for 32768 of them).
+        const auto key = [&](uint64_t i) { return (kinds[i] << 8) | (kinds[i] <= kItDelta ? fbw[i] : 0u); };
+        std::vector<uint64_t> at((kBatchKinds << 8) + 1, 0);
+        for (uint64_t i = 0; i < n_cols; i++) {
+            at[key(i) + 1] += pieces(parts[i], kinds[i] == kItRle ? kBItemRuns : ib);
+            at[(kItRest << 8) + 1] += pieces(hc[i].n - hc[i].n_compr, kBItemRest);
+        }
+        for (size_t k = 1; k < at.size(); k++) at[k] += at[k - 1];
+        for (int k = 0; k <= kBatchKinds; k++) b->seg[k] = at[size_t(k) << 8];
+        const std::unique_ptr<BItem[]> items(new BItem[n_items]);
+        for (uint64_t i = 0; i < n_cols; i++) {
+            const unsigned per = kinds[i] == kItRle ? kBItemRuns : ib;
+            uint64_t &to = at[key(i)];
+            for (uint64_t s = 0; s < parts[i]; s += per)
+                items[to++] = BItem{uint32_t(i), kinds[i], s, uint32_t(minu(per, parts[i] - s)), 0,
+                                    kinds[i] == kItDelta ? first[i] + s / per
+                                    : kinds[i] == kItRle ? run_rows[first[i] + s / per] : 0};
+            uint64_t &rest = at[kItRest << 8];
+            for (uint64_t r = hc[i].n_compr; r < hc[i].n; r += kBItemRest)
+                items[rest++] = BItem{uint32_t(i), kItRest, r, uint32_t(minu(kBItemRest, hc[i].n - r)), 0, 0};
+        }
+        if (n_items)
+            MS_CUDA_TRY(cudaMemcpyAsync(b->d_items, items.get(), sizeof(BItem) * n_items, cudaMemcpyHostToDevice, st));
+        MS_CUDA_TRY(cudaStreamSynchronize(st));
     }
-    // kind segments of the sorted queue
-    for (int k = 0, i = 0; k <= kBatchKinds; k++) {
-        while (i < int(hi.size()) && int(hi[i].kind) < k) i++;
-        b->seg[k] = k == kBatchKinds ? hi.size() : uint64_t(i);
-    }
-    if (!hi.empty())
-        MS_CUDA_TRY(cudaMemcpyAsync(b->d_items, hi.data(), sizeof(BItem) * hi.size(), cudaMemcpyHostToDevice, st));
-    MS_CUDA_TRY(cudaStreamSynchronize(st));
     int rc = read_err(a, st);
     if (rc) return batch_fail(b, rc);
     rc = batch_set_attr(b->cfg);
     if (rc) return batch_fail(b, rc);
     *out = b;
     return MS_OK;
+}
+
+}  // namespace
+
+extern "C" int ms_gpu_batch_create(const ms_col *cols, const uint64_t *consts, uint64_t n_cols, int cmp, ms_arena *a,
+                                   ms_batch **out, void *stream) {
+    if (!out || !a || (n_cols && (!cols || !consts))) return ms_fail(MS_ERR_INVALID, "batch_create: null argument");
+    if (cmp < MS_CMP_EQ || cmp > MS_CMP_GE) return ms_fail(MS_ERR_INVALID, "batch_create: comparison");
+    *out = nullptr;
+    uint64_t n_blocks = 0;
+    for (uint64_t i = 0; i < n_cols; i++)
+        if (cols[i].format != MS_FMT_RLE && cols[i].format != MS_FMT_UNCOMPR) n_blocks += cols[i].count_values / kBlock;
+    const unsigned ib = item_blocks(n_blocks);
+    const uint64_t mark = a->used;
+    int rc = plan_batch(cols, consts, n_cols, cmp, ib, a, out, (cudaStream_t)stream);
+    if (rc == MS_ERR_NOMEM && ib < kBItemBlocks) {
+        // the most blocks per item: the smallest plan
+        a->used = mark;
+        rc = plan_batch(cols, consts, n_cols, cmp, kBItemBlocks, a, out, (cudaStream_t)stream);
+    }
+    return rc;
 }
 
 extern "C" int ms_gpu_batch_set_config(ms_batch *b, const ms_tuning *t) {

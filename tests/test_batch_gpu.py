@@ -222,3 +222,52 @@ def test_batch_item_sizes(ms, arena, orc, blocks):
     for i, v in enumerate(vals):
         assert (int(cnt[i]), int(s[i])) == seen[id(v)][1], (i, len(v), cols[i].format)
     b.close()
+
+
+def test_batch_plan_costs_no_more_than_a_run(ms, arena, orc):
+    """Planning 32768 items (256 columns of 2^20 rows) takes less than two
+    runs of the plan (three with a comparison sort of the items)."""
+    import time
+    import torch
+    cols = []
+    for s in range(8):
+        kind = ("static", "dvbp", "for")[s % 3]  # planned without a pass over the column
+        v, bw = _column(orc, kind, 1 << 20, 50 + s)
+        cols.append(ms.morph(ms.Column.from_numpy(v, arena), _fmt(ms, kind, bw)))
+    cols = [cols[i % 8] for i in range(256)]
+    plan, run = [], []
+    for _ in range(6):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        b = ms.Batch(cols, [1 << 10] * len(cols))
+        t1 = time.perf_counter()
+        b.run()
+        t2 = time.perf_counter()
+        b.run()
+        plan.append(t1 - t0)
+        run.append(min(t2 - t1, time.perf_counter() - t2))
+        assert b.info()["items"] == 32768
+        b.close()
+    assert min(plan) < 2 * min(run), (min(plan), min(run))
+
+
+def test_batch_plan_in_a_short_arena(ms, arena, orc):
+    """Where the plan of small items does not fit, the plan of the largest
+    items is made."""
+    cols = [ms.morph(ms.Column.from_numpy(orc.uniform_bits(s, 9, 1 << 16), arena), ms.dynamic_vbp_f) for s in range(4)]
+    cols = [cols[i % 4] for i in range(64)]
+    want = [_expect(orc, orc.uniform_bits(s, 9, 1 << 16), 100) for s in range(4)]
+    made = []
+    for kb in range(4, 80):
+        a = ms.Arena(kb << 10)
+        try:
+            b = ms.Batch(cols, [100] * 64, arena=a)
+        except ms.MorphStoreError as e:
+            assert e.status == 4
+        else:
+            made.append(b.info()["items"])
+            cnt, s = b.run()
+            assert [(int(c), int(x)) for c, x in zip(cnt, s)] == [want[i % 4] for i in range(64)]
+            b.close()
+        a.close()
+    assert made[0] == 64 * 4 and made[-1] == 64 * 16 and made == sorted(made)
