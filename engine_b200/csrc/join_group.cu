@@ -964,8 +964,9 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
     const uint64_t sf = gr_in ? minu(cv.sfrom, gv.sfrom) : cv.sfrom;
     const bool binary = gr_in != nullptr;
     // 2^16 slots hold 2^15 groups; fewer when the column cannot have as many
-    // groups or the arena is short.  A size that was found too small is not
-    // tried again, so the table is filled once per size at most.
+    // groups or the arena is short.  A size that was found too small (below
+    // `least`) is not tried again, so the table is filled once per size at
+    // most.
     uint64_t cap = 1024, least = cap;
     while (cap < (uint64_t(1) << 16) && cap < 2 * n) cap <<= 1;
     const uint64_t mark = a->used;
@@ -1011,26 +1012,39 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
         }
         if (rc) return rc;
         const uint64_t groups = *h_groups;
-        uint64_t *ext = arena_take_t<uint64_t>(a, groups + 1);
-        uint64_t *gr = arena_take_t<uint64_t>(a, n + 1);
-        if (!ext || !gr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (group output)");
+        // the smallest table of that many groups, when it is smaller
+        const auto shrink = [&] {
+            while (least < 2 * groups) least <<= 1;
+            if (cap == least) return false;
+            cap = least;
+            return true;
+        };
+        // The outputs, and for the ranking a list of few groups or flags per
+        // row.  If neither fits beside the outputs, or their compressed form
+        // does not, the call is made again with a smaller table.
+        uint64_t *ext = arena_take_t<uint64_t>(a, groups + 1), *gr = arena_take_t<uint64_t>(a, n + 1);
+        const uint64_t nwords = (n + 31) / 32;
+        ulonglong2 *list = groups && groups <= kRankGroups ? arena_take_t<ulonglong2>(a, groups) : nullptr;
+        uint32_t *flags = nullptr, *wcnt = nullptr;
+        uint64_t *woff = nullptr, *tot = nullptr, *scr = nullptr;
+        if (groups && !list) {
+            flags = arena_take_t<uint32_t>(a, nwords + 1);
+            wcnt = arena_take_t<uint32_t>(a, nwords + 1);
+            woff = arena_take_t<uint64_t>(a, nwords + 1);
+            tot = arena_take_t<uint64_t>(a, 1);
+            scr = arena_take_t<uint64_t>(a, scan_scratch_words(nwords, 1));
+        }
+        if (!ext || !gr || (groups && !list && (!flags || !wcnt || !woff || !tot || !scr))) {
+            if (shrink()) continue;
+            return ms_fail(MS_ERR_NOMEM, "arena exhausted (group output)");
+        }
         const unsigned tgrid = unsigned(minu((cap + 255) / 256, persistent_grid(256, 8)));
-        ulonglong2 *list = nullptr;
-        if (groups && groups <= kRankGroups) {
-            list = arena_take_t<ulonglong2>(a, groups);
-            if (!list) return ms_fail(MS_ERR_NOMEM, "arena exhausted (group list)");
+        if (list) {
             k_group_list<<<tgrid, 256, 0, st>>>(t, sf, words + 1, list);
             k_group_rank<<<unsigned((groups + 31) / 32), 256, 0, st>>>(t, list, unsigned(groups), ext);
             MS_CUDA_TRY(cudaGetLastError());
         } else if (groups) {
             // first rows -> flags -> ranks
-            const uint64_t nwords = (n + 31) / 32;
-            uint32_t *flags = arena_take_t<uint32_t>(a, nwords + 1);
-            uint32_t *wcnt = arena_take_t<uint32_t>(a, nwords + 1);
-            uint64_t *woff = arena_take_t<uint64_t>(a, nwords + 1);
-            uint64_t *tot = arena_take_t<uint64_t>(a, 1);
-            uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(nwords, 1));
-            if (!flags || !wcnt || !woff || !tot || !scr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (group flags)");
             MS_CUDA_TRY(cudaMemsetAsync(flags, 0, 4 * (nwords + 1), st));
             k_group_list<<<tgrid, 256, 0, st>>>(t, sf, words + 1, nullptr);
             k_group_flags<<<tgrid, 256, 0, st>>>(t, flags);
@@ -1060,8 +1074,9 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
         const uint64_t n_scal_groups = *h_scal;
         const uint64_t n_scal_rows = n - sf;
         rc = write_values(gr, n - n_scal_rows, n_scal_rows, gr_format, 0, out_gr, a, st);
-        if (rc) return rc;
-        return write_values(ext, groups - n_scal_groups, n_scal_groups, ext_format, 0, out_ext, a, st);
+        if (!rc) rc = write_values(ext, groups - n_scal_groups, n_scal_groups, ext_format, 0, out_ext, a, st);
+        if (rc == MS_ERR_NOMEM && shrink()) continue;
+        return rc;
     }
 }
 

@@ -417,3 +417,26 @@ def test_positions_of_few_hits_in_a_short_arena(ms, orc, op):
         best.append(min(times))
         a.close()
     assert best[0] < 3 * best[1], best
+
+
+@pytest.mark.parametrize("groups,spare", [(100, 160), (3000, 330), (5000, 520)])
+@pytest.mark.parametrize("binary", [False, True])
+@pytest.mark.parametrize("code", [O.UNCOMPR, O.DYNAMIC_VBP])
+def test_group_table_gives_way_to_the_output(ms, orc, groups, spare, binary, code):
+    """Room for the output, the smallest table of the groups and flags per row
+    is enough, although the first table would fit without the output."""
+    n = 1 << 18
+    v = orc.uniform_bits(groups, 40, n) % np.uint64(groups)
+    g = v % np.uint64(7)
+    compressed = int(8.25 * (n + groups)) + (64 << 10) if code == O.DYNAMIC_VBP else 0
+    a = ms.Arena((2 if binary else 1) * 8 * n + 8 * n + compressed + ((spare + (160 if binary else 0)) << 10))
+    big = ms.Arena(64 << 20)
+    try:
+        cols = [ms.Column.from_numpy(v, a)] + ([ms.Column.from_numpy(g, a)] if binary else [])
+        gr, ext = ms.group(*cols, gr_f=F(ms, code), ext_f=F(ms, code))
+        egr, eext = orc.group(v, g) if binary else orc.group(v)
+        gr.arena = ext.arena = big  # for the values on the host
+        assert np.array_equal(gr.to_numpy(), egr) and np.array_equal(ext.to_numpy(), eext)
+    finally:
+        a.close()
+        big.close()
