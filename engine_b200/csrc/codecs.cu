@@ -397,6 +397,7 @@ __global__ void __launch_bounds__(256, 3) k_decode_delta(ColView c, DeltaSegs g,
 // rows, mean run 32: 149 us (208 with a look-back by CTAs that load, search,
 // look back and write one after another; 87 at the copy rate); runs of one
 // row 350 us a call (373), of 1000 rows 188 us (226).
+template <unsigned kStride>
 __global__ void __launch_bounds__(kRdThreads, 1)
     k_rle_encode(const uint64_t *__restrict__ in, uint64_t n, unsigned *words, ulonglong2 *__restrict__ out,
                  uint64_t *__restrict__ d_runs, unsigned *err) {
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(kRdThreads, 1)
     if (threadIdx.x == 0) {
         for (unsigned r = 0; r < kRdBufs; r++) load(r);
     }
-    RdPrefix<true> pre(words, ntiles);
+    RdPrefix<true, kStride> pre(words, ntiles);
     for (unsigned r = 0; r <= rounds + 1; r++) {
         const uint64_t t = tile_of(r);
         if (first_half && t < ntiles) {
@@ -453,7 +454,7 @@ __global__ void __launch_bounds__(kRdThreads, 1)
                     c += s_cnt[i];
                     z = max(z, s_last[i]);
                 }
-                rd_publish(words, t, c, z);
+                rd_publish<kStride>(words, t, c, z);
             }
         }
         if (!first_half && r && r <= rounds) pre.request(r - 1, tid);  // read in the next round
@@ -537,20 +538,19 @@ __global__ void __launch_bounds__(kRdThreads, 1)
 // A tile's published count carries the flag in its low two bits (0: nothing
 // yet, kRleFlagAgg: the tile's own rows, kRleFlagInc: the rows of tiles [0,
 // this tile]): written and read whole, so no fence is needed.  It has a cache
-// line of its own (rounds.cuh).
+// line of its own (rounds.cuh) unless the arena is short: `stride` words from
+// one tile's to the next.
 enum : unsigned { kRleFlagAgg = 1, kRleFlagInc = 2 };
-struct __align__(128) RleTileState {
-    unsigned long long r;
-};
+constexpr unsigned kRleStateStride = 16;
 
-__device__ __forceinline__ void rle_publish(RleTileState *s, unsigned flag, uint64_t rows) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&s->r), "l"((rows << 2) | flag) : "memory");
+__device__ __forceinline__ void rle_publish(unsigned long long *s, unsigned flag, uint64_t rows) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(s), "l"((rows << 2) | flag) : "memory");
 }
 
 // Warp-wide look-back (warp 0 of the tile): lane i inspects tile j - i, 32
 // predecessors per step; the nearest one with an inclusive count ends the
 // walk.  Returns false if a predecessor never published (bounded spin).
-__device__ bool rle_lookback(const RleTileState *state, uint64_t tile, uint64_t &excl) {
+__device__ bool rle_lookback(const unsigned long long *state, unsigned stride, uint64_t tile, uint64_t &excl) {
     const unsigned lane = threadIdx.x & 31u;
     excl = 0;
     for (int64_t j = int64_t(tile) - 1; j >= 0; j -= 32) {
@@ -558,7 +558,7 @@ __device__ bool rle_lookback(const RleTileState *state, uint64_t tile, uint64_t 
         unsigned long long r = kRleFlagInc;  // lanes before tile 0 act as an empty inclusive prefix
         if (me >= 0) {
             for (unsigned spins = 0; spins < kSpinLimit; spins++) {
-                asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(r) : "l"(&state[me].r) : "memory");
+                asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(r) : "l"(state + me * stride) : "memory");
                 if (r & 3u) break;
             }
         }
@@ -782,9 +782,9 @@ constexpr uint64_t kRleLbMaxMean = 4;
 __host__ __device__ constexpr unsigned rle_lb_slot(unsigned i) { return i + (i >> 3); }
 
 __global__ void __launch_bounds__(kRleLbThreads, 2) k_rle_expand_lb(const uint64_t *__restrict__ pairs,
-                                                                   uint64_t runs, uint64_t n, RleTileState *state,
-                                                                   unsigned *ticket, uint64_t *__restrict__ out,
-                                                                   unsigned *err) {
+                                                                   uint64_t runs, uint64_t n, unsigned long long *state,
+                                                                   unsigned stride, unsigned *ticket,
+                                                                   uint64_t *__restrict__ out, unsigned *err) {
     constexpr unsigned NW = kRleLbThreads / 32, NWD = kRleLbWin / 32;
     extern __shared__ __align__(128) uint8_t rle_smem[];
     // the tile's pairs, then (value, start within the tile) of its non-empty runs
@@ -857,11 +857,11 @@ __global__ void __launch_bounds__(kRleLbThreads, 2) k_rle_expand_lb(const uint64
         }
     }
     // publish the tile's rows, then the rows before it
-    RleTileState *me = state + tile;
+    unsigned long long *me = state + tile * stride;
     if (threadIdx.x == 0 && tile > 0) rle_publish(me, kRleFlagAgg, agg);
     if (wid == 0) {
         uint64_t excl = 0;
-        if (tile > 0 && !rle_lookback(state, tile, excl) && lane == 0) atomicOr(err, kErrTimeout);
+        if (tile > 0 && !rle_lookback(state, stride, tile, excl) && lane == 0) atomicOr(err, kErrTimeout);
         if (lane == 0) {
             rle_publish(me, kRleFlagInc, excl + agg);
             s_base = excl;
@@ -987,15 +987,20 @@ static int launch_rounds(void (*kern)(P...), uint64_t ntiles, cudaStream_t st, A
 }
 
 static int encode_rle(const uint64_t *d_in, uint64_t n, ms_col *out, ms_arena *a, cudaStream_t st) {
-    const uint64_t tiles = (n + kRdRows - 1) / kRdRows, nwords = tiles * kRdWordStride;
+    const uint64_t tiles = (n + kRdRows - 1) / kRdRows;
     uint8_t *data = arena_take_t<uint8_t>(a, 16 * n + 64);
-    unsigned *words = arena_take_t<unsigned>(a, nwords + 2);  // and the number of runs
+    // a line per word if there is room, else side by side; and the number of runs
+    uint64_t nwords = tiles * kRdWordStride;
+    unsigned *words = arena_take_t<unsigned>(a, nwords + 2);
+    const bool lines = words;
+    if (!lines) words = arena_take_t<unsigned>(a, (nwords = (tiles + 1) / 2 * 2) + 2);
     if (!data || !words) return ms_fail(MS_ERR_NOMEM, "arena exhausted (rle)");
     uint64_t runs = 0;
     if (n) {
         uint64_t *d_runs = reinterpret_cast<uint64_t *>(words + nwords);
         MS_CUDA_TRY(cudaMemsetAsync(words, 0, 4 * (nwords + 2), st));
-        int rc = launch_rounds(k_rle_encode, tiles, st, d_in, n, words, (ulonglong2 *)data, d_runs, a->d_err);
+        int rc = launch_rounds(lines ? k_rle_encode<kRdWordStride> : k_rle_encode<1>, tiles, st, d_in, n, words,
+                               (ulonglong2 *)data, d_runs, a->d_err);
         if (rc) return rc;
         ReadBack back(a, st);
         const uint64_t *h_runs = back.add(d_runs);
@@ -1020,14 +1025,17 @@ static int decode_rle(const ms_col *in, uint64_t *d_out, ms_arena *a, cudaStream
     if (n <= kRleLbMaxMean * runs && (reinterpret_cast<uintptr_t>(in->data) & 15u) == 0) {
         // short runs: one pass with a look-back
         const uint64_t tiles = (runs + kRleLbTile - 1) / kRleLbTile;
-        RleTileState *state = arena_take_t<RleTileState>(a, tiles + 1);
         unsigned *ticket = arena_take_t<unsigned>(a, 2);
+        // a line per state if there is room, else side by side
+        unsigned stride = kRleStateStride;
+        unsigned long long *state = arena_take_t<unsigned long long>(a, tiles * stride);
+        if (!state) state = arena_take_t<unsigned long long>(a, tiles * (stride = 1));
         if (!state || !ticket) return ms_fail(MS_ERR_NOMEM, "arena exhausted (rle decode)");
-        MS_CUDA_TRY(cudaMemsetAsync(state, 0, sizeof(RleTileState) * tiles, st));
+        MS_CUDA_TRY(cudaMemsetAsync(state, 0, 8 * tiles * stride, st));
         MS_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));
         constexpr size_t smem = size_t(rle_lb_slot(kRleLbTile)) * 16;
         MS_CUDA_TRY(cudaFuncSetAttribute(k_rle_expand_lb, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        k_rle_expand_lb<<<unsigned(tiles), kRleLbThreads, smem, st>>>((const uint64_t *)in->data, runs, n, state,
+        k_rle_expand_lb<<<unsigned(tiles), kRleLbThreads, smem, st>>>((const uint64_t *)in->data, runs, n, state, stride,
                                                                       ticket, d_out, a->d_err);
         MS_CUDA_TRY(cudaGetLastError());
         return MS_OK;

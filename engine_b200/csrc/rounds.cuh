@@ -80,11 +80,12 @@ __device__ __forceinline__ void rd_load(uint8_t *buf, uint64_t *full, const uint
 // line made a word some 5 us late: the line is written by many SMs while
 // others read it): bit 0 set, above it 13 bits that are summed up (block
 // widths, runs) and 13 bits of which the latest counts (last run head + 1, 0
-// for none).
+// for none).  kStride: words from one tile's to the next.
 constexpr unsigned kRdWordStride = 32;
+template <unsigned kStride = kRdWordStride>
 __device__ __forceinline__ void rd_publish(unsigned *words, uint64_t tile, unsigned sum, unsigned last) {
     const unsigned payload = last << 13 | sum;
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(words + tile * kRdWordStride), "r"(payload << 1 | 1u)
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(words + tile * kStride), "r"(payload << 1 | 1u)
                  : "memory");
 }
 __device__ __forceinline__ unsigned rd_peek(const unsigned *w) {
@@ -96,7 +97,7 @@ __device__ __forceinline__ unsigned rd_peek(const unsigned *w) {
 // What a tile needs from the words before it, by the output half: `base` =
 // the sum over the rounds before, `lower` = over the round's tiles before the
 // CTA's; kLast: `last` = the latest position before the tile (row + 1).
-template <bool kLast>
+template <bool kLast, unsigned kStride = kRdWordStride>
 struct RdPrefix {
     const unsigned *words;
     uint64_t ntiles;
@@ -112,7 +113,7 @@ struct RdPrefix {
         return unsigned(minu(gridDim.x, ntiles - uint64_t(r) * gridDim.x));
     }
     __device__ __forceinline__ const unsigned *word(unsigned r, unsigned i) const {
-        return words + (uint64_t(r) * gridDim.x + i) * kRdWordStride;
+        return words + (uint64_t(r) * gridDim.x + i) * kStride;
     }
     // requests round r's words; they are read by the next call of sums
     __device__ __forceinline__ void request(unsigned r, unsigned tid) {

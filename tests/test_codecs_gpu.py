@@ -308,3 +308,22 @@ def test_encoders_on_a_part_of_the_sms(ms, arena, orc, fmt):
         torch.cuda.synchronize()
         assert driver.cuStreamDestroy(stream)[0] == driver.CUresult.CUDA_SUCCESS
         assert driver.cuGreenCtxDestroy(green)[0] == driver.CUresult.CUDA_SUCCESS
+
+
+@pytest.mark.parametrize("mean_log2", [0, 3])
+def test_rle_in_a_short_arena(ms, orc, mean_log2):
+    """Room for the largest result and 12 KB: the words and states that tiles
+    publish lie side by side instead of in a line each."""
+    n = 3 * 148 * 6144 + 31
+    v = orc.runs(n, mean_log2, 20, n) if mean_log2 else orc.uniform_bits(n, 20, n)
+    a, b = ms.Arena(8 * n + 16 * n + (12 << 10)), ms.Arena(8 * n + (12 << 10))
+    try:
+        c = ms.morph(ms.Column.from_numpy(v, a), ms.rle_f)
+        want, m = orc.compress(O.RLE, 0, v)
+        assert c.meta() == m
+        assert np.array_equal(c.raw_bytes(), want[: m[1]])
+        c.arena = b
+        assert np.array_equal(c.to_numpy(), v)
+    finally:
+        a.close()
+        b.close()
