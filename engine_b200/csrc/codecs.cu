@@ -1045,12 +1045,12 @@ static int decode_rle(const ms_col *in, uint64_t *d_out, ms_arena *a, cudaStream
     uint64_t *trows = arena_take_t<uint64_t>(a, tiles + 1);
     uint64_t *tfirst = arena_take_t<uint64_t>(a, tiles + 1);
     uint64_t *tot = arena_take_t<uint64_t>(a, 1);
-    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(tiles, 1));
+    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(tiles));
     if (!trows || !tfirst || !tot || !scr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (rle decode)");
     const uint64_t *pairs = (const uint64_t *)in->data;
     k_rle_tile_rows<<<unsigned(tiles), kRleThreads, 0, st>>>(pairs, runs, tr, trows);
     MS_CUDA_TRY(cudaGetLastError());
-    MS_CUDA_TRY((scan_exclusive<uint64_t, 1>(trows, tiles, tfirst, tot, scr, st)));
+    MS_CUDA_TRY(scan_exclusive<uint64_t>(trows, tiles, tfirst, tot, scr, st));
     const uint64_t chunks = (n + kRleRows - 1) / kRleRows;
     uint32_t *ctile = arena_take_t<uint32_t>(a, chunks + 1);
     if (!ctile) return ms_fail(MS_ERR_NOMEM, "arena exhausted (rle decode)");

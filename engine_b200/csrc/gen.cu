@@ -115,11 +115,11 @@ extern "C" int ms_gpu_gen_sorted_gaps(uint64_t seed, const uint64_t *d_gap_table
     const uint64_t mark = a->used;
     uint64_t *gaps = arena_take_t<uint64_t>(a, n);
     uint64_t *tot = arena_take_t<uint64_t>(a, 1);
-    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(n, 1));
+    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(n));
     if (!gaps || !tot || !scr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (gen_sorted_gaps)");
     k_gap_draws<<<persistent_grid(256, 8), 256, 0, st>>>(seed, d_gap_table, n_table, n, gaps);
     MS_CUDA_TRY(cudaGetLastError());
-    MS_CUDA_TRY((scan_exclusive<uint64_t, 1>(gaps, n, d_out, tot, scr, st)));
+    MS_CUDA_TRY(scan_exclusive<uint64_t>(gaps, n, d_out, tot, scr, st));
     k_add_inclusive<<<persistent_grid(256, 8), 256, 0, st>>>(gaps, n, d_out);
     MS_CUDA_TRY(cudaGetLastError());
     MS_CUDA_TRY(cudaStreamSynchronize(st));
@@ -138,11 +138,11 @@ extern "C" int ms_gpu_gen_runs(uint64_t seed, unsigned log2_mean_len, unsigned v
     uint32_t *head = arena_take_t<uint32_t>(a, n);
     uint64_t *excl = arena_take_t<uint64_t>(a, n);
     uint64_t *tot = arena_take_t<uint64_t>(a, 1);
-    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(n, 1));
+    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(n));
     if (!head || !excl || !tot || !scr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (gen_runs)");
     k_run_heads<<<persistent_grid(256, 8), 256, 0, st>>>(seed, log2_mean_len, n, head);
     MS_CUDA_TRY(cudaGetLastError());
-    MS_CUDA_TRY((scan_exclusive<uint32_t, 1>(head, n, excl, tot, scr, st)));
+    MS_CUDA_TRY(scan_exclusive<uint32_t>(head, n, excl, tot, scr, st));
     k_run_values<<<persistent_grid(256, 8), 256, 0, st>>>(seed, value_bits, head, excl, n, d_out);
     MS_CUDA_TRY(cudaGetLastError());
     MS_CUDA_TRY(cudaStreamSynchronize(st));

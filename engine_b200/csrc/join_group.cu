@@ -1032,7 +1032,7 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
             wcnt = arena_take_t<uint32_t>(a, nwords + 1);
             woff = arena_take_t<uint64_t>(a, nwords + 1);
             tot = arena_take_t<uint64_t>(a, 1);
-            scr = arena_take_t<uint64_t>(a, scan_scratch_words(nwords, 1));
+            scr = arena_take_t<uint64_t>(a, scan_scratch_words(nwords));
         }
         if (!ext || !gr || (groups && !list && (!flags || !wcnt || !woff || !tot || !scr))) {
             if (shrink()) continue;
@@ -1050,7 +1050,7 @@ extern "C" int ms_gpu_group(const ms_col *gr_in, const ms_col *in, int gr_format
             k_group_flags<<<tgrid, 256, 0, st>>>(t, flags);
             k_popc_words<<<persistent_grid(256, 8), 256, 0, st>>>(flags, nwords, wcnt);
             MS_CUDA_TRY(cudaGetLastError());
-            MS_CUDA_TRY((scan_exclusive<uint32_t, 1>(wcnt, nwords, woff, tot, scr, st)));
+            MS_CUDA_TRY(scan_exclusive<uint32_t>(wcnt, nwords, woff, tot, scr, st));
             k_group_extents<<<tgrid, 256, 0, st>>>(t, flags, woff, ext);
             MS_CUDA_TRY(cudaGetLastError());
         }

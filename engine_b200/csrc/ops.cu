@@ -213,14 +213,14 @@ static int select_positions(const ColView &x, const ColView &y, int cmp, uint64_
     uint32_t *bc = arena_take_t<uint32_t>(a, nbt + 1);
     uint64_t *bo = arena_take_t<uint64_t>(a, nbt + 1);
     uint64_t *tot = arena_take_t<uint64_t>(a, 2);
-    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(nbt, 1));
+    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(nbt));
     if (!bc || !bo || !tot || !scr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (select)");
     MS_CUDA_TRY(cudaMemsetAsync(tot, 0, 16, st));
     const unsigned grid = grid_for_blocks(nbt);
     if (nbt) {
         k_sps<true, false><<<grid, 256, 0, st>>>(x, x, cmp, val, nullptr, nullptr, bc, a->d_err);
         MS_CUDA_TRY(cudaGetLastError());
-        MS_CUDA_TRY((scan_exclusive<uint32_t, 1>(bc, nbt, bo, tot, scr, st)));
+        MS_CUDA_TRY(scan_exclusive<uint32_t>(bc, nbt, bo, tot, scr, st));
     }
     uint64_t total = 0;
     MS_CUDA_TRY(cudaMemcpyAsync(&total, tot, 8, cudaMemcpyDeviceToHost, st));
@@ -524,12 +524,12 @@ extern "C" int ms_gpu_select_noalloc(int cmp, uint64_t val, const ms_col *in, ui
         MS_CUDA_TRY(cudaMemsetAsync(d_out_count, 0, 8, st));
         return MS_OK;
     }
-    if (scan_scratch_words(nbt, 1) > kNoAllocScanWords)
+    if (scan_scratch_words(nbt) > kNoAllocScanWords)
         return ms_fail(MS_ERR_INVALID, "select_noalloc: scan scratch too small");
     const unsigned grid = grid_for_blocks(nbt);
     k_sps<true, false><<<grid, 256, 0, st>>>(x, x, cmp, val, nullptr, nullptr, counts, err);
     MS_CUDA_TRY(cudaGetLastError());
-    MS_CUDA_TRY((scan_exclusive<uint32_t, 1>(counts, nbt, offsets, d_out_count, scan_scr, st)));
+    MS_CUDA_TRY(scan_exclusive<uint32_t>(counts, nbt, offsets, d_out_count, scan_scr, st));
     k_select_write<false><<<grid, 256, 0, st>>>(x, x, cmp, val, offsets, d_out_pos, nullptr, scalar_hits, err);
     MS_CUDA_TRY(cudaGetLastError());
     return MS_OK;

@@ -789,7 +789,7 @@ extern "C" int ms_gpu_query3(const ms_col *filter, int cmp, uint64_t c, const ms
         uint32_t *hits = arena_take_t<uint32_t>(a, nbt + 1);
         uint64_t *boff = arena_take_t<uint64_t>(a, nbt + 1);
         uint64_t *tot = arena_take_t<uint64_t>(a, 1);
-        uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(nbt, 1));
+        uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(nbt));
         GTable gt{arena_take_t<unsigned long long>(a, slots), arena_take_t<unsigned long long>(a, slots),
                   arena_take_t<unsigned long long>(a, slots), slots - 1};
         unsigned long long *cnt = arena_take_t<unsigned long long>(a, 1);
@@ -823,7 +823,7 @@ extern "C" int ms_gpu_query3(const ms_col *filter, int cmp, uint64_t c, const ms
                 MS_CUDA_TRY(cudaGetLastError());
             }
             MS_CUDA_TRY(cudaEventRecord(g_q3_ev[1], st));
-            MS_CUDA_TRY((scan_exclusive<uint32_t, 1>(hits, nbt, boff, tot, scr, st)));
+            MS_CUDA_TRY(scan_exclusive<uint32_t>(hits, nbt, boff, tot, scr, st));
             k_q3_extents<<<unsigned(minu(slots / 256, persistent_grid(256, 2))), 256, 0, st>>>(
                 gt, fv, kv, cmp, c, bits, lo, span, boff, cnt, out, a->d_err);
             MS_CUDA_TRY(cudaGetLastError());

@@ -556,11 +556,11 @@ extern "C" int ms_gpu_bwi_compress(const uint64_t *d_in, uint64_t nblk, const vo
     uint64_t *sz = arena_take_t<uint64_t>(a, nblk + 1);
     uint64_t *off = arena_take_t<uint64_t>(a, nblk + 1);
     uint64_t *tot = arena_take_t<uint64_t>(a, 1);
-    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(nblk, 1));
+    uint64_t *scr = arena_take_t<uint64_t>(a, scan_scratch_words(nblk));
     if (!sz || !off || !tot || !scr) return ms_fail(MS_ERR_NOMEM, "arena exhausted (bwi)");
     k_bwi_sizes<<<sel_grid(nblk), 256, 0, st>>>((const BlockStats *)d_stats, d_choice, nblk, sz);
     MS_CUDA_TRY(cudaGetLastError());
-    MS_CUDA_TRY((scan_exclusive<uint64_t, 1>(sz, nblk, off, tot, scr, st)));
+    MS_CUDA_TRY(scan_exclusive<uint64_t>(sz, nblk, off, tot, scr, st));
     uint64_t bytes = 0;
     if (nblk) {
         ReadBack back(a, st);
