@@ -50,9 +50,12 @@ struct GTable {  // global group table (open addressing)
 __device__ __forceinline__ bool gtable_add(const GTable &t, uint64_t key, uint64_t first, uint64_t sum) {
     uint64_t h = qhash(key) & t.mask;
     for (uint64_t p = 0; p <= t.mask; p++) {
-        const unsigned long long old = atomicCAS(t.keys + h, kQEmpty, key);
-        if (old == kQEmpty || old == key) {
-            atomicMin(t.first + h, first);
+        // A key that is there with a smaller row costs two loads and one
+        // atomic: rows beyond a CTA's table come here one by one.
+        unsigned long long x = ((volatile unsigned long long *)t.keys)[h];
+        if (x == kQEmpty) x = atomicCAS(t.keys + h, kQEmpty, key);
+        if (x == kQEmpty || x == key) {
+            if (first < ((volatile unsigned long long *)t.first)[h]) atomicMin(t.first + h, first);
             atomicAdd(t.sums + h, sum);
             return true;
         }
@@ -404,7 +407,7 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
         const uint64_t *const maux = meas.fmt == MS_FMT_FOR_DVBP ? meas.aux : nullptr;
         QWarp &mine = s_warp[cw];
         unsigned queued = 0;  // rows in the warp's queue
-        unsigned turn = 0;    // pairs of the tiles before, mod W
+        unsigned turn = 0;    // units of the tiles before, mod W
         for (unsigned t = 0;; t++) {
             const unsigned st = t % S, use = t / S;
             if (!mbar_wait(full + st, use & 1u)) {
@@ -414,13 +417,20 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
             const unsigned T = desc[st].nblk;
             if (T == 0) break;
             const uint64_t b0 = desc[st].b0;
-            const unsigned pairs = (T + 1) / 2;
+            // One block at a time where the ring's pairs are fewer than the
+            // warps: wide columns have three blocks to a tile, and with pairs
+            // 6 of 16 warps worked (2^23 rows, three columns of 64 bits, 90 %
+            // kept, 1000 groups: 647 us, 506 with single blocks).  Else pairs:
+            // a single block's filter takes half the lanes (2^27 rows, 10 %
+            // kept: 624 us a call, 532 with pairs).
+            const bool two = S * ((T + 1) / 2) >= W;
+            const unsigned units = two ? (T + 1) / 2 : T;
             const uint32_t *o = offs + st * kQCols * kQTile;
             const uint8_t *w = bws + st * kQCols * kQTile;
-            for (unsigned pr = (cw + W - turn) % W; pr < pairs; pr += W) {
-                const unsigned j = 2 * pr + hb;
+            for (unsigned u = (cw + W - turn) % W; u < units; u += W) {
+                const unsigned j0 = two ? 2 * u : u, j = j0 + hb;
                 unsigned m = 0;
-                if (j < T) {
+                if (j < T && (two || !hb)) {
                     m = mask32_block_rt(w[j], reinterpret_cast<const uint64_t *>(ring + o[j]), l, h, pred, bad);
                     if (w[kQTile + j] - 1u >= 64u || w[2 * kQTile + j] - 1u >= 64u || w[3 * kQTile + j] - 1u >= 64u) {
                         bad = true;
@@ -450,7 +460,7 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
                     for (unsigned i = 0; i < 4; i++) {
                         const bool in = h0 + 32u * i + lane < hits;
                         e[i] = in ? mine.hits[h0 + 32u * i + lane] : 0u;
-                        const unsigned jj = 2 * pr + (e[i] >> 9);
+                        const unsigned jj = j0 + (e[i] >> 9);
                         uint64_t v = vbp_extract(reinterpret_cast<const uint64_t *>(ring + o[kQTile + jj]), w[kQTile + jj],
                                                  e[i] & 511u);
                         if (kaux) v += __ldg(kaux + ((b0 + jj) >> 1));
@@ -476,12 +486,12 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
                     }
                     __syncwarp();
                 }
-                if (lane < 2 && 2 * pr + lane < T) blk_hits[b0 + 2 * pr + lane] = lane ? alive - alive0 : alive0;
+                if (lane <= unsigned(two) && j0 + lane < T) blk_hits[b0 + j0 + lane] = lane ? alive - alive0 : alive0;
                 // their group keys and measures
                 for (unsigned a0 = 0; a0 < alive; a0 += 32) {
                     const unsigned cnt = min(32u, alive - a0);
                     if (lane < cnt) {
-                        const unsigned ee = mine.hits[a0 + lane], jj = 2 * pr + (ee >> 9), row = ee & 511u;
+                        const unsigned ee = mine.hits[a0 + lane], jj = j0 + (ee >> 9), row = ee & 511u;
                         const uint64_t blk = b0 + jj;
                         uint64_t g = vbp_extract(reinterpret_cast<const uint64_t *>(ring + o[2 * kQTile + jj]),
                                                  w[2 * kQTile + jj], row);
@@ -509,7 +519,7 @@ __global__ void __launch_bounds__(32 * (W + 1), 1)
                 }
                 __syncwarp();  // the list is free for the next pair
             }
-            turn = (turn + pairs) % W;
+            turn = (turn + units) % W;
             __syncwarp();
             if (lane == 0) mbar_arrive(empty + st);
         }

@@ -206,3 +206,45 @@ def test_query3_equals_gpu_operator_pipeline(ms, arena, orc):
     assert np.array_equal(keys, gk)
     assert np.array_equal(e2, ext.to_numpy())
     assert np.array_equal(sums, s.to_numpy())
+
+
+@pytest.mark.parametrize("widths", [(64, 64, 64, 64), (10, 64, 16, 64), (33, 40, 20, 20), (12, 12, 12, 12)])
+@pytest.mark.parametrize("groups", [7, 5000])
+@pytest.mark.parametrize("n", [512 * 3 + 1, 512 * 148 * 9 - 5, 400_009])
+def test_query3_tiles_of_few_and_many_blocks(ms, arena, orc, widths, groups, n):
+    """Tiles of 3 to 32 blocks, taken one by one or in pairs; nearly all rows
+    kept; more groups than a CTA's table holds."""
+    filt, fk, gkey, meas = (orc.uniform_bits(s, 12, n) << np.uint64(max(w - 12, 0)) for s, w in enumerate(widths, 71))
+    filt, fk = filt >> np.uint64(1), (fk >> np.uint64(max(widths[1] - 12, 0)))
+    if widths[1] > 12:
+        fk = fk + np.uint64((1 << widths[1]) - (1 << 13))  # keys of the column's width
+    gkey = (orc.uniform_bits(9, 40, n) % np.uint64(groups)) << np.uint64(max(widths[2] - 13, 0))
+    lk = np.unique(fk)[::2]
+    c = int(np.sort(filt)[int(0.9 * n)])
+    cols = [_col(ms, arena, orc, v, O.DYNAMIC_VBP) for v in (filt, fk, gkey, meas)]
+    keys, ext, sums, npos = ms.query3(cols[0], O.CMP_LT, c, cols[1], ms.Column.from_numpy(lk, arena), cols[2], cols[3])
+    ek, ee, es, enp = _expect(orc, O.CMP_LT, c, filt, fk, gkey, meas, lk, orc.scalar_from(O.DYNAMIC_VBP, 0, cols[0].meta()))
+    assert npos == enp
+    assert np.array_equal(keys, ek) and np.array_equal(ext, ee) and np.array_equal(sums, es)
+
+
+def test_query3_keeps_its_warps_busy_on_wide_columns(ms, arena, orc):
+    """2^23 rows, nine of ten kept: 64-bit columns (three blocks to a tile) cost
+    at most a third more than 16-bit ones (1.5 times as much with tiles shared
+    out in pairs of blocks: 6 of 16 warps)."""
+    import time
+    n = 1 << 23
+    filt, fk, meas = orc.uniform_bits(1, 12, n), orc.uniform_bits(2, 16, n), orc.uniform_bits(3, 16, n)
+    gkey = orc.uniform_bits(4, 40, n) % np.uint64(1000)
+    lk = ms.Column.from_numpy(np.arange(0, 1 << 16, 2, dtype=np.uint64), arena)
+    best = []
+    for wide in (False, True):
+        cols = [ms.Column.from_numpy(v, arena) if wide and i in (1, 3) else
+                ms.morph(ms.Column.from_numpy(v, arena), ms.dynamic_vbp_f) for i, v in enumerate((filt, fk, gkey, meas))]
+        times = []
+        for _ in range(12):
+            t0 = time.perf_counter()
+            ms.query3(cols[0], O.CMP_LT, 3686, cols[1], lk, cols[2], cols[3])
+            times.append(time.perf_counter() - t0)
+        best.append(min(times))
+    assert best[1] < 4 / 3 * best[0], best
