@@ -628,9 +628,10 @@ void batch_release(ms_batch *b) {
 // few items the first grab empties the queue and the launch ends on whichever
 // warp drew the slow ones.  The item is halved, down to 8 blocks, until there
 // are 8 items for each of 16 warps per SM.  256 columns (5.6 k items of 32
-// blocks): 225 us with 32 blocks per item, 125 with 16, 118
-// with 8, 142 with 4, where the queue atomics and the per-item setup show.
-// Thousands of columns keep the 32 that their setup is spread over.
+// blocks), a graph replay with its results: 297 us with 32 blocks per item,
+// 182 with 16, 171 with 8, 190 with 4, where the queue atomics and the
+// per-item setup show.  Thousands of columns keep the 32 that their setup is
+// spread over.
 unsigned item_blocks(uint64_t n_blocks) {
     unsigned ib = kBItemBlocks;
     while (ib > 8 && n_blocks / ib < 8ull * 16 * sm_count()) ib /= 2;

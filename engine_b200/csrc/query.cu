@@ -50,12 +50,14 @@ struct GTable {  // global group table (open addressing)
 __device__ __forceinline__ bool gtable_add(const GTable &t, uint64_t key, uint64_t first, uint64_t sum) {
     uint64_t h = qhash(key) & t.mask;
     for (uint64_t p = 0; p <= t.mask; p++) {
-        // A key that is there with a smaller row costs two loads and one
-        // atomic: rows beyond a CTA's table come here one by one.
+        // A key that is there with a smaller row costs two loads (taken
+        // together) and one atomic: rows beyond a CTA's table come here one by
+        // one.
         unsigned long long x = ((volatile unsigned long long *)t.keys)[h];
+        const unsigned long long f = ((volatile unsigned long long *)t.first)[h];
         if (x == kQEmpty) x = atomicCAS(t.keys + h, kQEmpty, key);
         if (x == kQEmpty || x == key) {
-            if (first < ((volatile unsigned long long *)t.first)[h]) atomicMin(t.first + h, first);
+            if (first < f) atomicMin(t.first + h, first);
             atomicAdd(t.sums + h, sum);
             return true;
         }
