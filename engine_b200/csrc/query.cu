@@ -47,14 +47,19 @@ struct GTable {  // global group table (open addressing)
     uint64_t mask;
 };
 
+// kLook: reads the slot before changing it, so that a key that is there with a
+// smaller row costs two loads and one atomic instead of three atomics -- for
+// rows that come one by one.  The flush of a CTA's groups meets mostly empty
+// slots, or slots that other CTAs are filling, and does not look.
+template <bool kLook = false>
 __device__ __forceinline__ bool gtable_add(const GTable &t, uint64_t key, uint64_t first, uint64_t sum) {
     uint64_t h = qhash(key) & t.mask;
     for (uint64_t p = 0; p <= t.mask; p++) {
-        // A key that is there with a smaller row costs two loads (taken
-        // together) and one atomic: rows beyond a CTA's table come here one by
-        // one.
-        unsigned long long x = ((volatile unsigned long long *)t.keys)[h];
-        const unsigned long long f = ((volatile unsigned long long *)t.first)[h];
+        unsigned long long x = kQEmpty, f = ~0ull;
+        if (kLook) {
+            x = ((volatile unsigned long long *)t.keys)[h];
+            f = ((volatile unsigned long long *)t.first)[h];
+        }
         if (x == kQEmpty) x = atomicCAS(t.keys + h, kQEmpty, key);
         if (x == kQEmpty || x == key) {
             if (first < f) atomicMin(t.first + h, first);
@@ -64,6 +69,13 @@ __device__ __forceinline__ bool gtable_add(const GTable &t, uint64_t key, uint64
         h = (h + 1) & t.mask;
     }
     return false;
+}
+
+// For rows beyond a CTA's table.  Out of line: inlined into the consumers' loop
+// it made the pass slower, 2^27 rows that all find their group in the table
+// 301 us instead of 282.
+__device__ __noinline__ bool gtable_look(const GTable &t, uint64_t key, uint64_t first, uint64_t sum) {
+    return gtable_add<true>(t, key, first, sum);
 }
 
 __global__ void __launch_bounds__(256) k_query3(ColView filt, ColView fk, ColView gkey, ColView meas, int cmp,
@@ -162,7 +174,7 @@ __global__ void __launch_bounds__(256) k_query3(ColView filt, ColView fk, ColVie
 // together and queued per warp, and 32 queued rows at a time go to the CTA's
 // group table.  The producer takes block locations from windows it loaded
 // ahead (window.cuh) and forms a tile before it waits for its stage: its path
-// per tile bounded the pass.  2^27 rows: 293 us (356 before; 412 with the
+// per tile bounded the pass.  2^27 rows: 282 us (356 before; 412 with the
 // listed hits alone), of which reading the columns takes 149; the rest is the
 // consumers' instructions at 17 warps per SM (24 warps leave a smaller ring:
 // 383 us).
@@ -218,7 +230,7 @@ __device__ __forceinline__ bool qtable_add(const QTable &t, const GTable &gt, ui
             h = (h + 1) & (kQSlots - 1);
         }
     }
-    return gtable_add(gt, key, row, val);
+    return gtable_look(gt, key, row, val);
 }
 
 // value of row r (0..511) of a vbp block of width bw staged in shared memory;
